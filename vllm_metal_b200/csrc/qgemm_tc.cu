@@ -843,12 +843,16 @@ static int dispatch_g(const HostArgs& a, cudaStream_t st) {
     return a.prepacked ? launch_stream<T, BITS, G, 64, BITS == 4>(a, ksplit, st)
                        : launch_stream<T, BITS, G, 64, false>(a, ksplit, st);
   }
+  // Many rows: the dequantised tile goes to tensor memory here too.  With it in shared memory a 128 x 256 tile moves about 208 B a
+  // cycle through shared memory at full tensor rate (products' reads of both operands 96, x fill 64, dequantised writes 32, packed
+  // words 16) where 128 fit: measured 0.62 of the rate.  In tensor memory 144 B remain: int4, M = 2048, 6144 x 4096 98 -> 85 us,
+  // 28672 x 4096 447 -> 392 us, 4096 x 14336 212 -> 188 us; M = 128 29 -> 21 us; int8 51200 x 5120 1062 -> 1014 us.
   if (a.prepacked && BITS == 4) {
-    if (a.M <= 128) return launch_cfg<T, BITS, G, 128, 3, 3, 8, false, BITS == 4>(a, 1, st);
-    return launch_cfg<T, BITS, G, 256, 2, 3, 8, false, BITS == 4>(a, 1, st);
+    if (a.M <= 128) return launch_cfg<T, BITS, G, 128, 3, 4, 8, false, BITS == 4, true>(a, 1, st);
+    return launch_cfg<T, BITS, G, 256, 3, 5, 8, false, BITS == 4, true>(a, 1, st);
   }
-  if (a.M <= 128) return launch_cfg<T, BITS, G, 128, 3, 3, 8>(a, 1, st);
-  return launch_cfg<T, BITS, G, 256, 2, 3, 8>(a, 1, st);
+  if (a.M <= 128) return launch_cfg<T, BITS, G, 128, 3, 4, 8, false, false, true>(a, 1, st);
+  return launch_cfg<T, BITS, G, 256, 3, 5, 8, false, false, true>(a, 1, st);
 }
 
 template <typename T, int BITS>
