@@ -235,6 +235,65 @@ int b200_qlinear_experts(const void* x, const uint32_t* w, const void* scales, c
                          int group_size, int bits, int x_dtype, int dtype, int sb_dtype, int64_t x_stride,
                          int64_t y_stride, void* stream);
 
+/* The same for all experts at once, without a host read-back (csrc/qexperts.cu): bf16 activations, scales, biases and bias; k and
+ * n_out whole multiples of 64; operands 16-byte aligned and contiguous.
+ *   b200_qexpert_route   logits = x . w^T (+ bias) in fp32, rounded to bf16; the `top` largest, best first, ties to the lower
+ *                        number (NaN before all), to chosen [rows, top]; scores: softmax over the chosen ones, or with over_all = 1
+ *                        over all experts before the choice, norm = 1: divided by their sum.  At most 128 experts, top <= 32.
+ *   b200_expert_plan     (b200_hybrid_ops.h) with tile_rows = b200_qexpert_tile_rows(...) -- the smaller one, if several
+ *                        products share a plan; 0: the products do not take these sizes.
+ *   b200_qexpert_rows    y [total, cols] fp16 (saturated) = x[pairs[i] / top]; `permute` (4-bit weights): every eight columns in the
+ *                        order 0 4 1 5 2 6 3 7, as the products expect theirs
+ *   b200_qexpert_product gated = 1: out[i, :] (fp16, same column order as x) = act(gate, up) of row i, both rounded to bf16;
+ *                        activation 0 silu(g) u, 1 clipped SwiGLU (alpha 1.702, limit 7).  gated = 0: out[pairs[i], :] (bf16).
+ *   b200_qexpert_sum     out [rows, cols] = sum_j weights[row, j] y[row * top + j, :], fp32 sums in the order of j
+ *   b200_qexpert_failed  synchronises; 1 if a plan did not fit together or a bounded wait ran out (results invalid), else 0 */
+typedef struct b200_qexpert_product_args {
+  const void* x;      /* fp16 [total, k], sorted by expert */
+  const uint32_t* w;  /* [experts, n_out, k * bits / 32] */
+  const void* scales; /* bf16 [experts, n_out, k / group_size] */
+  const void* biases;
+  const void* bias; /* bf16 [experts, n_out] or NULL */
+  const uint32_t* up_w; /* gated: the other half; else NULL */
+  const void* up_scales;
+  const void* up_biases;
+  const void* up_bias;
+  void* out; /* [total, n_out] */
+  const int32_t* pairs;
+  const int32_t* first;
+  const int32_t* tiles;
+  int32_t total, experts, n_out, k, bits, group_size, tile_rows, gated, activation;
+} b200_qexpert_product_args;
+int b200_qexpert_route(const void* x, const void* w, const void* bias, int32_t* chosen, float* scores, int rows, int width,
+                       int experts, int top, int64_t x_stride, int over_all, int norm, void* stream);
+int b200_qexpert_tile_rows(int rows, int top, int experts, int n_out, int k, int group_size, int gated);
+int b200_qexpert_rows(const void* x, const int32_t* pairs, void* y, int total, int top, int cols, int64_t x_stride, int permute,
+                      void* stream);
+int b200_qexpert_product(const b200_qexpert_product_args* a, void* stream);
+int b200_qexpert_sum(const void* y, const float* weights, void* out, int rows, int top, int cols, void* stream);
+int b200_qexpert_failed(void);
+/* All of it in one call: out [rows, width] = the block's result for x [rows, width] (bf16, x_stride elements apart).  The router is
+ * bf16 [experts, width].  B200_ERR_UNSUPPORTED for sizes that the parts above do not take (nothing was enqueued). */
+typedef struct b200_qexpert_matrix {
+  const uint32_t* w;
+  const void* scales;
+  const void* biases;
+  const void* bias;
+} b200_qexpert_matrix;
+typedef struct b200_qexpert_block_args {
+  const void* x;
+  const void* router_w;
+  const void* router_bias;
+  b200_qexpert_matrix gate, up, down;
+  void* out;
+  void* workspace; /* b200_qexpert_block_workspace_bytes, 256-byte aligned */
+  size_t workspace_bytes;
+  int64_t x_stride;
+  int32_t rows, width, ff, experts, top, bits, group_size, activation, over_all, norm;
+} b200_qexpert_block_args;
+size_t b200_qexpert_block_workspace_bytes(int rows, int width, int ff, int experts, int top);
+int b200_qexpert_block(const b200_qexpert_block_args* a, void* stream);
+
 /* Test / tuning knob: which kernel b200_qlinear runs.  0 = auto (tcgen05 + TMEM + TMA kernel
  * whenever the shape qualifies, else the mma.sync kernel), 1 = always the mma.sync kernel,
  * 2 = tcgen05 kernel or B200_ERR_UNSUPPORTED.  Process-wide; returns 0 on success. */

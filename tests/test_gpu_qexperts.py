@@ -1,0 +1,110 @@
+"""The grouped quantized expert kernels (csrc/qexperts.cu) against float64 over their ranges' edges."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _values(m, e):
+    """float64 values of an expert's affine weights."""
+    w = m.weight[e].to(torch.int64) & 0xFFFFFFFF
+    q = (w.unsqueeze(-1) >> (torch.arange(32 // m.bits, device=w.device) * m.bits)) & (2**m.bits - 1)
+    q = q.flatten(-2).unflatten(-1, (-1, m.group_size)).double()
+    return (q * m.scales[e].double().unsqueeze(-1) + m.biases[e].double().unsqueeze(-1)).flatten(-2)
+
+
+def _block(hidden, inter, experts, top, bits, group, act, routing, bias, down_bits=None):
+    from vllm_metal_b200.quant.switch_linear import MoEBlock, QuantizedSwitchLinear, Router, SwitchGLU
+
+    g = torch.Generator(device="cuda").manual_seed(hidden + inter + bits)
+    glu = SwitchGLU(hidden, inter, experts, bias, group, bits, torch.bfloat16, "cuda", activation=act)
+    for name, n, k, b in (("gate_proj", inter, hidden, bits), ("up_proj", inter, hidden, bits), ("down_proj", hidden, inter, down_bits or bits)):
+        dense = torch.randn((experts, n, k), device="cuda", generator=g) * k**-0.5
+        extra = torch.randn((experts, n), device="cuda", generator=g) * 0.1 if bias else None
+        setattr(glu, name, QuantizedSwitchLinear.from_dense(dense, extra, group, b, torch.bfloat16))
+    router = Router(hidden, experts, bias, torch.bfloat16, "cuda")
+    router.weight.copy_(torch.randn((experts, hidden), device="cuda", generator=g) * 2 * hidden**-0.5)
+    return MoEBlock(router, glu, top, routing)
+
+
+@pytest.mark.parametrize("tokens", [1, 15, 17, 64, 65, 192, 193, 500])
+@pytest.mark.parametrize("bits,group,hidden,inter,top,act,routing,bias,down_bits", [
+    (4, 64, 320, 192, 2, "gpt_oss", "topk_softmax", True, 4),   # odd rows of groups; half a tile of features on the way out
+    (4, 32, 576, 448, 3, "silu", "softmax_topk", False, 8),     # a way out of other words than the way in
+    (8, 128, 1024, 128, 1, "silu", "softmax_topk", False, 8),
+    (8, 32, 4096, 64, 2, "silu", "topk_softmax", True, 8),      # scales of one item only fit beside large tiles
+])
+def test_grouped_block_vs_float64(tokens, bits, group, hidden, inter, top, act, routing, bias, down_bits):
+    from vllm_metal_b200.metal import get_ops
+
+    blk = _block(hidden, inter, 7, top, bits, group, act, routing, bias, down_bits)
+    x = torch.randn((tokens, hidden), device="cuda", generator=torch.Generator(device="cuda").manual_seed(tokens)).bfloat16()
+    before = get_ops().launches
+    y = blk(x)
+    assert get_ops().launches - before == 6  # route, plan, rows, two products, sum
+    idx, scores = blk.route(x)
+    # the choice: the block says fp32 logits rounded to bf16, ties to the lowest
+    logits = blk.router(x).float()
+    vals = torch.softmax(logits, -1) if routing == "softmax_topk" else logits
+    best, want = torch.sort(vals, dim=-1, descending=True, stable=True)
+    same = (idx == want[:, :top]).all(1)
+    assert same.float().mean() >= 0.98  # a logit on the edge of two bf16 values may go either way
+    part = torch.softmax(best[:, :top], -1) if routing == "topk_softmax" else best[:, :top] / best[:, :top].sum(-1, keepdim=True)
+    off = ((scores[same] - part[same]).abs() / part[same]).double()
+    # sums in another order put a logit now and then on the other side of a rounding edge: one step of bf16, 2^-8 of it
+    assert (off <= 2e-5).double().mean() >= 0.98 and off.max() <= 2 * 2**-8 * float(logits.abs().max()) + 2e-5
+    glu, ref = blk.experts, torch.zeros((tokens, hidden), dtype=torch.float64, device="cuda")
+    for e in range(7):
+        at, place = (idx == e).nonzero(as_tuple=True)
+        if len(at):
+            lin = lambda z, m, e=e: z @ _values(m, e).T + (m.bias[e].double() if bias else 0)  # noqa: E731
+            g, u = lin(x[at].double(), glu.gate_proj), lin(x[at].double(), glu.up_proj)
+            if act == "gpt_oss":
+                g, u = g.clamp(max=7.0), u.clamp(-7.0, 7.0)
+                h = g * torch.sigmoid(1.702 * g) * (u + 1)
+            else:
+                h = torch.nn.functional.silu(g) * u
+            ref[at] += lin(h, glu.down_proj) * scores[at, place].double()[:, None]
+    # four roundings to bf16 (gate, up, activation, result: 2^-9 each at most, a third of it in the mean) and weights of 11 bits
+    assert (y.double() - ref).norm() <= 4 * 2**-9 * ref.norm()
+    assert not get_ops().qexpert_failed()
+
+
+def test_choices_of_ties_and_nan():
+    """Ties go to the lowest expert; a row of NaN stays in range, as the sort of the general path has it."""
+    blk = _block(64, 64, 7, 3, 4, 64, "silu", "topk_softmax", False)
+    blk.router.weight.zero_()
+    x = torch.randn((5, 64), device="cuda").bfloat16()
+    x[3] = float("nan")
+    idx, scores = blk.route(x)
+    assert idx.tolist() == [[0, 1, 2]] * 5 and idx.dtype == torch.int64
+    assert torch.isnan(scores[3]).all() and torch.allclose(scores[:3], torch.full((3, 3), 1 / 3, device="cuda"))
+
+
+def test_indices_out_of_range_are_refused():
+    blk = _block(64, 64, 7, 2, 4, 64, "silu", "topk_softmax", False)
+    x = torch.randn((3, 64), device="cuda").bfloat16()
+    for bad in (-1, 7):
+        idx = torch.zeros((3, 2), dtype=torch.int64, device="cuda")
+        idx[1, 1] = bad
+        with pytest.raises((ValueError, RuntimeError)):
+            blk.experts(x, idx)
+
+
+@pytest.mark.parametrize("top,tokens", [(2, 33), (7, 5)])
+def test_the_parts_and_the_whole_agree(top, tokens):
+    """The block in one call and its parts one by one (as with a trace, or rows that cannot be read in 16-byte units)."""
+    blk = _block(320, 192, 7, top, 4, 64, "gpt_oss", "topk_softmax", True)
+    x = torch.randn((tokens, 2, 320), device="cuda").bfloat16()[:, 1]  # rows apart
+    y = blk(x)
+    blk.trace = []
+    assert torch.equal(blk(x), y) and len(blk.trace) == 1
+    wide = torch.nn.functional.pad(x, (1, 0))[:, 1:]  # rows that start off 16 bytes: copied
+    torch.testing.assert_close(blk(wide), y)
+    idx, scores = blk.route(x)
+    parts = blk.experts(x, idx)
+    want = (parts.float() * scores[..., None]).sum(1)
+    torch.testing.assert_close(y.float(), want, rtol=2**-7, atol=1e-5)

@@ -79,11 +79,32 @@ __device__ __forceinline__ bool mbar_wait_or_fail(uint32_t bar, uint32_t parity)
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
+// The same for a warp that waits long (see mbar_wait_parked).
+__device__ __forceinline__ bool mbar_wait_parked_or_fail(uint32_t bar, uint32_t parity) {
+  for (uint32_t spins = 0; spins < (1u << 20); ++spins) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(2000u)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar,
                                             int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
 __device__ __forceinline__ void fence_proxy_async() {
@@ -128,6 +149,16 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
       : "memory");
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
+// The same store without the wait: issue several, then tmem_st_wait() once.
+__device__ __forceinline__ void tmem_st16_nowait(uint32_t taddr, const uint32_t* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // One lane of a converged warp.  Code under `if (elect_one())` keeps warp-uniform operands (descriptors, tensor
 // memory addresses) provably uniform for the compiler; issuing under `if (lane == 0)` instead measured ~80 cycles
 // per MMA issue.
@@ -254,6 +285,22 @@ inline int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* ptr
   return B200_OK;
 }
 
+// A matrix [rows, slabs * width] seen as [slabs][rows][width]: one copy brings the same rows of several neighbouring slabs.
+inline int make_map_slabs(CUtensorMap* map, CUtensorMapDataType dt, const void* ptr, uint64_t width, uint64_t rows, uint64_t slabs,
+                          uint64_t elem_bytes, uint64_t row_stride_bytes, uint32_t box_rows, uint32_t box_slabs,
+                          CUtensorMapL2promotion promo) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return set_error(B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  cuuint64_t dims[3] = {width, rows, slabs};
+  cuuint64_t strides[2] = {row_stride_bytes, width * elem_bytes};
+  cuuint32_t box[3] = {(cuuint32_t)width, box_rows, box_slabs};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult rc = fn(map, dt, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, promo, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (rc != CUDA_SUCCESS)
+    return set_error(B200_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)rc);
+  return B200_OK;
+}
 
 }  // namespace tc
 }  // namespace b200

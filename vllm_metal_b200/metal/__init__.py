@@ -90,6 +90,31 @@ class PagedAttnArgs(ctypes.Structure):
     ]
 
 
+class QExpertProductArgs(ctypes.Structure):
+    """Mirror of ``b200_qexpert_product_args``."""
+
+    _fields_ = [(n, ctypes.c_void_p) for n in ("x", "w", "scales", "biases", "bias", "up_w", "up_scales", "up_biases", "up_bias",
+                                               "out", "pairs", "first", "tiles")]
+    _fields_ += [(n, ctypes.c_int32) for n in ("total", "experts", "n_out", "k", "bits", "group_size", "tile_rows", "gated",
+                                               "activation")]
+
+
+class QExpertMatrix(ctypes.Structure):
+    """Mirror of ``b200_qexpert_matrix``."""
+
+    _fields_ = [(n, ctypes.c_void_p) for n in ("w", "scales", "biases", "bias")]
+
+
+class QExpertBlockArgs(ctypes.Structure):
+    """Mirror of ``b200_qexpert_block_args``."""
+
+    _fields_ = [("x", ctypes.c_void_p), ("router_w", ctypes.c_void_p), ("router_bias", ctypes.c_void_p), ("gate", QExpertMatrix),
+                ("up", QExpertMatrix), ("down", QExpertMatrix), ("out", ctypes.c_void_p), ("workspace", ctypes.c_void_p),
+                ("workspace_bytes", ctypes.c_size_t), ("x_stride", ctypes.c_int64)]
+    _fields_ += [(n, ctypes.c_int32) for n in ("rows", "width", "ff", "experts", "top", "bits", "group_size", "activation",
+                                               "over_all", "norm")]
+
+
 # Every symbol include/*.h declares; the CPU test-suite checks the library
 # exports all of them (tests/test_host_logic.py::test_library_exports_every_declared_symbol).
 EXPORTED_SYMBOLS = (
@@ -107,6 +132,14 @@ EXPORTED_SYMBOLS = (
     "b200_paged_attention_static_scratch",
     "b200_qlinear",
     "b200_qlinear_experts",
+    "b200_qexpert_route",
+    "b200_qexpert_tile_rows",
+    "b200_qexpert_rows",
+    "b200_qexpert_product",
+    "b200_qexpert_sum",
+    "b200_qexpert_failed",
+    "b200_qexpert_block",
+    "b200_qexpert_block_workspace_bytes",
     "b200_qlinear_prepack",
     "b200_qlinear_prepacked",
     "b200_set_qlinear_variant",
@@ -224,6 +257,13 @@ def load_library() -> ctypes.CDLL:
     lib.b200_qlinear_prepacked.argtypes = lib.b200_qlinear.argtypes
     lib.b200_qlinear_experts.argtypes = [vp, vp, vp, vp, vp, vp, ctypes.POINTER(ctypes.c_int32), i32, i32, i32, i32, i32,
                                          i32, i32, i32, i64, i64, vp]
+    lib.b200_qexpert_route.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i64, i32, i32, vp]
+    lib.b200_qexpert_rows.argtypes = [vp, vp, vp, i32, i32, i32, i64, i32, vp]
+    lib.b200_qexpert_product.argtypes = [ctypes.POINTER(QExpertProductArgs), vp]
+    lib.b200_qexpert_block.argtypes = [ctypes.POINTER(QExpertBlockArgs), vp]
+    lib.b200_qexpert_block_workspace_bytes.argtypes = [i32] * 5
+    lib.b200_qexpert_block_workspace_bytes.restype = ctypes.c_size_t
+    lib.b200_qexpert_sum.argtypes = [vp, vp, vp, i32, i32, i32, vp]
     lib.b200_qlinear_prepack.argtypes = [vp, vp, i32, i32, i32, i32, vp]
     lib.b200_dequantize_rows.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp]
     lib.b200_qstream_blob_bytes.restype = ctypes.c_int64
@@ -610,6 +650,74 @@ class _Ops(HybridOps):
         self._check(rc)
         self.launches += sum(1 for c in counts if c)
         return out
+
+    # -- all experts of a quantized block at once (csrc/qexperts.cu) ------------------------------
+    def qexpert_route(self, x, weight, bias, top: int, over_all: bool, norm: bool):
+        """``(chosen int32 [T, top], scores fp32 [T, top])`` of bf16 ``x [T, H]`` (rows of whole 16-byte units) and a bf16
+        router ``weight [E, H]``."""
+        t, width = x.shape
+        chosen = torch.empty((t, top), dtype=torch.int32, device=x.device)
+        scores = torch.empty((t, top), dtype=torch.float32, device=x.device)
+        self._check(self._lib.b200_qexpert_route(x.data_ptr(), weight.data_ptr(), _ptr(bias), chosen.data_ptr(), scores.data_ptr(), t,
+                                                 width, weight.shape[0], top, x.stride(0), int(over_all), int(norm), _stream()))
+        self.launches += 1
+        return chosen, scores
+
+    def qexpert_tile_rows(self, rows: int, top: int, experts: int, n_out: int, k: int, group_size: int, gated: bool) -> int:
+        return self._lib.b200_qexpert_tile_rows(rows, top, experts, n_out, k, group_size, int(gated))
+
+    def qexpert_rows(self, x, pairs, top: int, bits: int):
+        y = torch.empty((pairs.shape[0], x.shape[1]), dtype=torch.float16, device=x.device)
+        self._check(self._lib.b200_qexpert_rows(x.data_ptr(), pairs.data_ptr(), y.data_ptr(), pairs.shape[0], top, x.shape[1],
+                                                x.stride(0), int(bits == 4), _stream()))
+        self.launches += 1
+        return y
+
+    def qexpert_product(self, x, lin, plan, up=None, activation: int = 0):
+        """``lin``, ``up``: anything with the tensors of a ``QuantizedSwitchLinear``.  With ``up`` the way in (fp16, sorted),
+        else the way out (bf16, by pair)."""
+        pairs, first, tiles, tile_rows = plan
+        e, n, _ = lin.weight.shape
+        a = QExpertProductArgs()
+        a.x, a.w, a.scales, a.biases, a.bias = (_ptr(t) for t in (x, lin.weight, lin.scales, lin.biases, lin.bias))
+        if up is not None:
+            a.up_w, a.up_scales, a.up_biases, a.up_bias = (_ptr(t) for t in (up.weight, up.scales, up.biases, up.bias))
+        out = torch.empty((x.shape[0], n), dtype=torch.bfloat16 if up is None else torch.float16, device=x.device)
+        a.out, a.pairs, a.first, a.tiles = (_ptr(t) for t in (out, pairs, first, tiles))
+        a.total, a.experts, a.n_out, a.k = x.shape[0], e, n, x.shape[1]
+        a.bits, a.group_size, a.tile_rows, a.gated, a.activation = lin.bits, lin.group_size, tile_rows, int(up is not None), activation
+        self._check(self._lib.b200_qexpert_product(ctypes.byref(a), _stream()))
+        self.launches += 1
+        return out
+
+    def qexpert_sum(self, y, scores):
+        t, top = scores.shape
+        out = torch.empty((t, y.shape[1]), dtype=torch.bfloat16, device=y.device)
+        self._check(self._lib.b200_qexpert_sum(y.data_ptr(), scores.data_ptr(), out.data_ptr(), t, top, y.shape[1], _stream()))
+        self.launches += 1
+        return out
+
+    def qexpert_block(self, x, router, matrices, bits: int, group_size: int, top: int, activation: int, over_all: bool, norm: bool):
+        """The whole block in one call: ``router`` (weight, bias), ``matrices`` (weight, scales, biases, bias) of gate, up and down.
+        ``None`` if the grouped kernels do not take these sizes."""
+        t, width = x.shape
+        e, ff = matrices[0][1].shape[:2]
+        nbytes = self._lib.b200_qexpert_block_workspace_bytes(t, width, ff, e, top)
+        out = torch.empty((t, width), dtype=torch.bfloat16, device=x.device)
+        ws = torch.empty((nbytes,), dtype=torch.uint8, device=x.device)
+        mats = [QExpertMatrix(*(None if p is None else p.data_ptr() for p in m)) for m in matrices]
+        a = QExpertBlockArgs(x.data_ptr(), router[0].data_ptr(), _ptr(router[1]), *mats, out.data_ptr(), ws.data_ptr(), nbytes, x.stride(0),
+                             t, width, ff, e, top, bits, group_size, activation, over_all, norm)
+        rc = self._lib.b200_qexpert_block(ctypes.byref(a), _stream())
+        if rc == _ERR_UNSUPPORTED:
+            return None
+        self._check(rc)
+        self.launches += 6
+        return out
+
+    def qexpert_failed(self) -> bool:
+        """Whether a wait inside the grouped product kernel ever ran out (synchronises)."""
+        return self._lib.b200_qexpert_failed() != 0
 
     def qlinear_prepack(self, w, bits: int = 4, inverse: bool = False, out=None):
         """Load-time repack of an MLX-layout packed weight into the streaming layout (same shape)."""

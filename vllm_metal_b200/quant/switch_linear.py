@@ -6,12 +6,14 @@ projections are ``QuantizedSwitchLinear`` modules -- named in vllm_metal/quant/a
 expert weights ``[E, N, K*bits/32]`` (third-party arithmetic: mlx 0.32.0 / mlx-lm 254d153, not under
 /root/reference -> parity unpinned, semantics restated in oracle/moe.py).  Same attribute names and shapes here.
 
-B200 form: the (token, expert) pairs are sorted by expert and every expert that received rows runs ONE affine
-quantized GEMM over its gathered rows through the same kernels as the dense linears (`b200_qlinear_experts`: one
-C-ABI call per projection that loops over the experts): each
-expert's weights are streamed once per step however many tokens picked it.  The per-expert row counts are read back
-to the host once per block (one small D2H copy): this is the functional path of row N2 -- launch-bound at decode
-batch sizes (3 x experts-hit launches per layer); a grouped persistent kernel is the next step and is not built.
+B200 form: choice of the experts, the sort of the (token, expert) pairs, ONE launch of the gate and up products of all
+experts with the activation in their epilogue, ONE of the down products, the weighted sum (csrc/qexperts.cu).  Nothing is read
+back to the host.  A block of 32 experts of 2880 x 2880, top 4, int4: 172 us for 32 tokens and 313 us for 1024, where a GEMM per
+expert and projection with a read-back of the counts took 1205 and 2745.
+
+Sizes and types that those kernels do not take (``SwitchGLU.grouped_tile_rows``), and the ``mx.gather_qmm`` form of a single
+projection, run one affine quantized GEMM per expert that received rows (`b200_qlinear_experts`), with the row counts read back
+once.
 """
 
 from __future__ import annotations
@@ -146,6 +148,8 @@ def _act_gpt_oss(gate: torch.Tensor, up: torch.Tensor, alpha: float = 1.702, lim
 
 
 ACTIVATIONS = {"silu": _act_silu, "gpt_oss": _act_gpt_oss}
+_GROUPED_ACTIVATIONS = {"silu": (_act_silu, 0), "gpt_oss": (_act_gpt_oss, 1)}  # those that the grouped kernels compute
+_WORDS = (torch.int32, torch.uint32)
 
 
 class SwitchGLU(nn.Module):
@@ -159,8 +163,53 @@ class SwitchGLU(nn.Module):
         self.gate_proj, self.up_proj, self.down_proj = mk(hidden, inter), mk(hidden, inter), mk(inter, hidden)
         self.activation = activation
 
+    def grouped_tile_rows(self, x: torch.Tensor, top: int) -> int:
+        """Rows per tile with which the grouped kernels take ``x [T, H]``, 0 if they do not.  They take bf16 rows and affine
+        parameters, widths that are multiples of 64 and 16-byte aligned tensors; gradients pass through the other path."""
+        g, u, d = self.gate_proj, self.up_proj, self.down_proj
+        if (x.dtype != torch.bfloat16 or not x.is_cuda or x.shape[0] == 0 or self.activation not in _GROUPED_ACTIVATIONS
+                or ACTIVATIONS[self.activation] is not _GROUPED_ACTIVATIONS[self.activation][0]
+                or (torch.is_grad_enabled() and x.requires_grad)):
+            return 0
+        ops = get_ops()
+        if getattr(ops, "_qlinear_kernel", 0) == 1 or (g.bits, g.group_size) != (u.bits, u.group_size):
+            return 0
+        e, h, f = g.num_experts, x.shape[1], g.out_features
+        rows = []
+        for m, n, k in ((g, f, h), (u, f, h), (d, h, f)):
+            group = m.group_size
+            if (m.bits not in (4, 8) or group not in (32, 64, 128) or k % 64 or k % group or m.weight.shape != (e, n, k * m.bits // 32)
+                    or m.scales.shape != (e, n, k // group) or m.biases.shape != m.scales.shape):
+                return 0
+            for t, dtypes in ((m.weight, _WORDS), (m.scales, (x.dtype,)), (m.biases, (x.dtype,)), (m.bias, (x.dtype,))):
+                if t is not None and (t.dtype not in dtypes or t.device != x.device or not t.is_contiguous() or t.data_ptr() % 16):
+                    return 0
+            if m.bias is not None and m.bias.shape != (e, n):
+                return 0
+            rows.append(ops.qexpert_tile_rows(x.shape[0], top, e, n, k, group, m is not d))
+        return min(rows)
+
+    def grouped(self, x: torch.Tensor, indices: torch.Tensor, tile_rows: int) -> torch.Tensor:
+        """``x [T, H]``, ``indices [T, k]`` int32, in range -> ``[T * k, H]``."""
+        ops = get_ops()
+        if x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
+            x = x.clone(memory_format=torch.contiguous_format)
+        plan = ops.expert_plan(indices.contiguous(), self.gate_proj.num_experts, tile_rows)
+        xs = ops.qexpert_rows(x, plan[0], indices.shape[1], self.gate_proj.bits)
+        h = ops.qexpert_product(xs, self.gate_proj, plan, up=self.up_proj, activation=_GROUPED_ACTIVATIONS[self.activation][1])
+        if (self.down_proj.bits == 4) != (self.gate_proj.bits == 4):  # the way in left the columns in its own weights' order
+            order = torch.tensor([0, 2, 4, 6, 1, 3, 5, 7] if self.gate_proj.bits == 4 else [0, 4, 1, 5, 2, 6, 3, 7], device=h.device)
+            h = h.view(h.shape[0], -1, 8)[:, :, order].reshape(h.shape)
+        return ops.qexpert_product(h, self.down_proj, plan)
+
     def forward(self, x: torch.Tensor, indices: torch.Tensor) -> torch.Tensor:
         t, k = indices.shape
+        tile_rows = self.grouped_tile_rows(x, k) if x.dim() == 2 and x.shape[0] == t and k else 0
+        if tile_rows:
+            lo, hi = (int(v) for v in torch.aminmax(indices))
+            if lo < 0 or hi >= self.gate_proj.num_experts:
+                raise ValueError(f"expert indices must lie in [0, {self.gate_proj.num_experts}), got {lo} .. {hi}")
+            return self.grouped(x, indices.to(torch.int32), tile_rows).reshape(t, k, -1)
         order, counts = _sort_pairs(indices, self.gate_proj.num_experts)
         token_of_pair = torch.div(order, k, rounding_mode="floor")
         xs = x.index_select(0, token_of_pair).contiguous()  # rows grouped by expert: gathered once for gate and up
@@ -209,7 +258,57 @@ class MoEBlock(nn.Module):
         self.routing, self.norm_topk_prob = routing, norm_topk_prob
         self.trace: list | None = None  # tests: a list collects (indices, scores) of every forward
 
+    def _choose(self, x: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor] | None:
+        """Router product and choice in one launch, ``(int32, fp32)`` of ``[T, k]``; ``None`` where it does not apply."""
+        r = self.router
+        if (type(r) is not Router or not x.is_cuda or x.dtype != torch.bfloat16 or x.shape[0] == 0
+                or (torch.is_grad_enabled() and x.requires_grad)):
+            return None
+        w, b = r.weight, r.bias
+        if (x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16 or x.shape[1] % 32 or w.shape[1] != x.shape[1] or w.dtype != x.dtype
+                or not w.is_contiguous() or w.data_ptr() % 16 or w.device != x.device or w.shape[0] > 128
+                or not 1 <= self.top_k <= min(32, w.shape[0])
+                or (b is not None and (b.dtype != x.dtype or not b.is_contiguous() or b.device != x.device))):
+            return None
+        return get_ops().qexpert_route(x, w, b, self.top_k, self.routing == "softmax_topk", self.norm_topk_prob)
+
+    def _whole(self, x: torch.Tensor) -> torch.Tensor | None:
+        """The block in one call, ``None`` where that does not apply (what is checked here: types, shapes and strides; sizes and
+        alignment by the call)."""
+        r, glu = self._modules["router"], self._modules["experts"]
+        act = _GROUPED_ACTIVATIONS.get(getattr(glu, "activation", None))
+        if (type(r) is not Router or type(glu) is not SwitchGLU or self.trace is not None or x.dtype != torch.bfloat16 or not x.is_cuda
+                or act is None or ACTIVATIONS[glu.activation] is not act[0] or x.shape[0] == 0 or x.stride(1) != 1
+                or (x.requires_grad and torch.is_grad_enabled())):
+            return None
+        ops, dev, h = get_ops(), x.device, x.shape[1]
+        if getattr(ops, "_qlinear_kernel", 0) == 1:
+            return None
+        lins = [glu._modules[n] for n in ("gate_proj", "up_proj", "down_proj")]
+        bits, group = lins[0].bits, lins[0].group_size
+        if bits not in (4, 8) or group not in (32, 64, 128) or any(type(m) is not QuantizedSwitchLinear or m.bits != bits or m.group_size != group
+                                                                   for m in lins):
+            return None
+        bufs = [(b["weight"], b["scales"], b["biases"], b.get("bias")) for b in (m._buffers for m in lins)]
+        e, f = bufs[0][1].shape[:2]
+        for (w, s, b, extra), n, k in zip(bufs, (f, f, h), (h, h, f), strict=True):
+            if (s.dtype is not torch.bfloat16 or b.dtype is not torch.bfloat16 or w.dtype not in _WORDS or s.shape != (e, n, k // group)
+                    or b.shape != s.shape or w.shape != (e, n, k * bits // 32) or w.device != dev or s.device != dev or b.device != dev
+                    or not (w.is_contiguous() and s.is_contiguous() and b.is_contiguous())):
+                return None
+            if extra is not None and (extra.dtype is not torch.bfloat16 or extra.shape != (e, n) or extra.device != dev
+                                      or not extra.is_contiguous()):
+                return None
+        rw, rb = r._buffers["weight"], r._buffers.get("bias")
+        if (rw.dtype is not torch.bfloat16 or rw.shape != (e, h) or rw.device != dev or not rw.is_contiguous() or (rb is not None and (
+                rb.dtype is not torch.bfloat16 or rb.shape != (e,) or rb.device != dev or not rb.is_contiguous()))):
+            return None
+        return ops.qexpert_block(x, (rw, rb), bufs, bits, group, self.top_k, act[1], self.routing == "softmax_topk", self.norm_topk_prob)
+
     def route(self, x: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+        got = self._choose(x) if x.dim() == 2 else None
+        if got is not None:
+            return got[0].to(torch.int64), got[1]
         logits = self.router(x).float()
         # stable descending sort: equal scores (bf16-rounded logits do tie) go to the lowest expert id, on every rank
         # and in the oracle alike -- torch.topk leaves the order of ties unspecified
@@ -226,9 +325,19 @@ class MoEBlock(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         lead = x.shape[:-1]
         x2 = x.reshape(-1, x.shape[-1])
-        idx, scores = self.route(x2)
+        y = self._whole(x2)
+        if y is not None:
+            return y.reshape(*lead, -1)
+        tile_rows = self.experts.grouped_tile_rows(x2, self.top_k) if isinstance(self.experts, SwitchGLU) else 0
+        got = self._choose(x2) if tile_rows else None
+        idx, scores = got if got is not None else self.route(x2)
         if self.trace is not None:
             self.trace.append((idx.cpu().numpy(), scores.cpu().numpy()))
+        if (tile_rows and scores.dtype == torch.float32 and not (torch.is_grad_enabled() and scores.requires_grad)
+                and type(self.router) in (Router, nn.Linear) and self.router.weight.shape[0] <= self.experts.gate_proj.num_experts):
+            # no more logits than there are experts: the choices are in range
+            y = self.experts.grouped(x2, idx.to(torch.int32), tile_rows)
+            return get_ops().qexpert_sum(y, scores.contiguous()).reshape(*lead, -1)
         y = self.experts(x2, idx)  # [T, k, hidden]
         out = (y.float() * scores[..., None]).sum(dim=1).to(x.dtype)
         return out.reshape(*lead, -1)
