@@ -21,6 +21,7 @@ from ...metal import get_ops
 from ...metal.constants import KERNEL_BLOCK_SIZES
 from ..caches.kv_cache import B200PagedKVCache
 from ..context import PagedAttentionContext
+from ...host_lists import as_int32, fill_rows
 
 
 # Test knob: False runs the reference's step-by-step sequence (norm, rope, reshape_and_cache as
@@ -51,14 +52,21 @@ def _build_block_tables_np(raw_block_tables: list[list[int]], cache_block_size: 
         return np.zeros((0, 0), dtype=np.int32), cache_block_size
     width = max(len(row) for row in raw_block_tables)
     table = np.zeros((len(raw_block_tables), width), dtype=np.int32)
-    for i, row in enumerate(raw_block_tables):
-        table[i, : len(row)] = row
+    fill_rows(table, raw_block_tables)
     if cache_block_size in KERNEL_BLOCK_SIZES:
         return table, cache_block_size
     kbs = _pick_kernel_block_size(cache_block_size)
     ratio = cache_block_size // kbs
     expanded = table[:, :, None] * ratio + np.arange(ratio, dtype=np.int32)
     return expanded.reshape(table.shape[0], -1).astype(np.int32), kbs
+
+
+def _as_int64(values) -> np.ndarray:
+    """Slots fit 32 bits in all but the largest caches: converted that way first."""
+    try:
+        return as_int32(values).astype(np.int64)
+    except OverflowError:
+        return np.asarray(values, dtype=np.int64)
 
 
 def _build_block_tables(raw_block_tables, cache_block_size, device="cuda"):
@@ -102,7 +110,7 @@ def _kernel_metadata(ctx, group_index, raw_slot_mapping, raw_block_tables, cache
     if meta is None:
         table, kbs = _build_block_tables_np(raw_block_tables, cache_block_size)
         meta = _KernelMetadata(
-            slot_mapping=_to_device(np.asarray(raw_slot_mapping, dtype=np.int64), torch.int64, device),
+            slot_mapping=_to_device(_as_int64(raw_slot_mapping), torch.int64, device),
             seq_lens=_to_device(np.asarray(ctx.context_lens, dtype=np.int32), torch.int32, device),
             cu_seqlens_q=_to_device(np.asarray(ctx.cu_seqlens, dtype=np.int32), torch.int32, device),
             block_tables=_to_device(table, torch.int32, device),
@@ -145,6 +153,7 @@ def sdpa_forward(
         sinks = sinks.float()
 
     cache_block_size = kv_cache.block_size_for_layer(layer_idx)
+    own_meta = meta is not None  # the caller's; else built from the context, whose cu_seqlens the device copy then is
     if meta is None:
         group_index = kv_cache.group_index_for_layer(layer_idx)
         if ctx.kv_groups is None:
@@ -226,11 +235,13 @@ def sdpa_forward(
     f16_out = plain_tail and q.dtype == torch.bfloat16 and (
         getattr(o_proj, "weight_blob", None) is not None or getattr(o_proj, "weight_tc", None) is not None)
     out = torch.empty((t, n_heads, cache_hd), dtype=torch.float16 if f16_out else q.dtype, device=q.device)
+    window = getattr(ctx, "verify_window_q", 1)
     ops.paged_attention_primitive(
         q, k_cache, v_cache, kv_cache.kv_heads_per_layer[layer_idx], float(scale), 0.0,
         meta.block_tables, meta.seq_lens, meta.cu_seqlens_q, meta.block_size, meta.max_seq_len,
         kv_cache.sliding_window_per_layer[layer_idx], out,
-        window_seqlen_q=getattr(ctx, "verify_window_q", 1), sinks=sinks)  # sdpa.py:713,730
+        window_seqlen_q=window, sinks=sinks,  # sdpa.py:713,730
+        **({"cu_seqlens_host": ctx.cu_seqlens} if window > 1 and not own_meta else {}))
     if hd < cache_hd:
         out = out[..., :hd]  # strip the pad before o_proj (truncate_padded_output)
     out = out.reshape(t, n_heads * hd)

@@ -60,6 +60,24 @@ def output_path(component: str | None = None) -> Path:
     return _PKG_DIR / (LIB_NAME if component is None else f"lib_b200_{component}_ops.so")
 
 
+def host_library_path() -> Path:
+    return _PKG_DIR / "lib_b200_host.so"
+
+
+def build_host(force: bool = False) -> Path:
+    """``csrc/host_lists.c`` with the C compiler, against this interpreter's headers."""
+    import sysconfig
+
+    out, src = host_library_path(), CSRC_DIR / "host_lists.c"
+    if not force and out.exists() and out.stat().st_mtime >= src.stat().st_mtime:
+        return out
+    cmd = [os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I", sysconfig.get_path("include"), "-o", str(out), str(src)]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed ({proc.returncode}) on {src.name}:\n{proc.stderr[-4000:]}")
+    return out
+
+
 def stamp_path(component: str | None = None) -> Path:
     out = output_path(component)
     return out.with_name(out.name + ".stamp")
@@ -124,6 +142,7 @@ def build(force: bool = False, verbose: bool = False, component: str | None = No
     from concurrent.futures import ThreadPoolExecutor
 
     out = output_path(component)
+    build_host(force)
     if not force and out.exists() and not stale_artifacts(component):
         return out
     extra = os.environ.get("B200_NVCC_EXTRA", "").split()  # tuning experiments (-DQGEMM_...), not for shipping

@@ -22,6 +22,7 @@ import torch
 from ..attention.context import clear_context, get_context, prepare_grouped, prepare_unified
 from ..attention.impls.sdpa import _KernelMetadata, _kernel_metadata
 from ..attention.impls.segments import SegmentMetadata
+from ..host_lists import as_int32, fill_rows
 from ..metal import get_ops
 from ..metal.constants import PARTITION_SIZE
 
@@ -157,7 +158,7 @@ class PagedModelRunner:
                 ctx.state_slots = list(state_slots)
             if rows is None:
                 rows = [c - 1 for c in ctx.cu_seqlens[1:]]
-            ids = torch.tensor(list(input_ids), dtype=torch.int32).pin_memory().to(self.device, non_blocking=True)
+            ids = torch.from_numpy(as_int32(list(input_ids))).pin_memory().to(self.device, non_blocking=True)
             row_ids = torch.tensor(list(rows), dtype=torch.int64).pin_memory().to(self.device, non_blocking=True)
             self.last_logits = self.model(ids, ctx, self.kv_cache, logits_rows=row_ids)
             # bytes that crossed PCIe for this step: ids + logit rows + the kernel metadata sdpa uploads once
@@ -212,7 +213,7 @@ class PagedModelRunner:
             prepare_unified(reqs, [], self.block_size, merge_verify_windows=self.merge_verify_windows)
         ctx = get_context()
         try:
-            ids = torch.tensor(list(input_ids), dtype=torch.int32).pin_memory().to(self.device, non_blocking=True)
+            ids = torch.from_numpy(as_int32(list(input_ids))).pin_memory().to(self.device, non_blocking=True)
             self.last_verify_logits = self.model(ids, ctx, self.kv_cache, logits_rows=None)
             toks = self._greedy(self.last_verify_logits).cpu().tolist()
             nseq = len(ctx.cu_seqlens) - 1
@@ -267,8 +268,7 @@ class PagedModelRunner:
         if isinstance(block_ids, np.ndarray):
             tables[:n, : block_ids.shape[1]] = block_ids
         else:
-            for i, ids in enumerate(block_ids):
-                tables[i, : len(ids)] = ids
+            fill_rows(tables, block_ids)
         blk = tables[np.arange(n), pos // self.block_size].astype(np.int64)
         b.np_view("slot_mapping")[:n] = blk * self.block_size + pos % self.block_size
         b.np_view("input_ids")[:n] = np.asarray(token_ids, dtype=np.int32)
