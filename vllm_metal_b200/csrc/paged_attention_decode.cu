@@ -63,7 +63,11 @@ int decode_window_rows(const b200_paged_attn_args& a) {
   return r < 1 ? 1 : (r > a.window_seqlen_q ? a.window_seqlen_q : r);
 }
 
-int launch_decode_mma(const b200_paged_attn_args& a, const SplitWorkspace* ws, cudaStream_t st, int skip_qlen) {
+bool decode_cluster_supported(const b200_paged_attn_args& a) {
+  return decode_mma_supported(a) && !wide_form(a) && keep_first(a) == 0 && !a.slopes && value_dim(a) == a.head_dim;
+}
+
+int launch_decode_mma(const b200_paged_attn_args& a, const SplitWorkspace* ws, cudaStream_t st, int skip_qlen, int cluster, int psize) {
   DecodeParams p{};
   p.out = a.out;
   p.query = a.query;
@@ -96,13 +100,15 @@ int launch_decode_mma(const b200_paged_attn_args& a, const SplitWorkspace* ws, c
   p.num_blocks = a.num_blocks;
   p.scale = a.scale;
   p.softcap = a.softcap;
-  p.partitioned = ws != nullptr;
+  p.partitioned = ws != nullptr || cluster > 0;
+  p.cluster = cluster;
   p.ws = SplitWorkspace{};
   if (ws) p.ws = *ws;
+  if (cluster > 0) p.ws.partition_size = psize;
   p.ws.skip_qlen = skip_qlen;
   p.ws.out_f16 = out_is_f16(a);
   p.ws.denom_eps = denom_eps(a);
-  dim3 grid(a.num_kv_heads, a.num_q_tokens, ws ? ws->num_partitions : 1);
+  dim3 grid(a.num_kv_heads, a.num_q_tokens, ws ? ws->num_partitions : cluster > 0 ? cluster : 1);
   p.win_rows = skip_qlen > 0 ? 1 : decode_window_rows(a);
   p.win_subs = 1;
   if (p.win_rows > 1) {  // one CTA per (sequence, sub-window of win_rows rows); paged_ops.cpp:508-515
