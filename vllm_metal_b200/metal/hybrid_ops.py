@@ -155,7 +155,8 @@ def _f32(name: str, t: torch.Tensor | None, n: int) -> int | None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the handle alone: building torch's Stream object takes some 4 us, for every launch
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 class HybridOps:
