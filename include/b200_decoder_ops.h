@@ -61,6 +61,9 @@ int b200_norm_rope_cache(void* q, void* k, const void* v, const void* q_norm_wei
 /* out[r, i] = silu(gate_up[r, i]) * gate_up[r, inter + i], i in [0, inter). */
 int b200_silu_mul(const void* gate_up, void* out, int rows, int inter,
                   int64_t in_stride, int64_t out_stride, int dtype, void* stream);
+/* The same for bf16 input, the bf16-rounded results stored as fp16 (saturated): the operand type of the quantized products. */
+int b200_silu_mul_f16(const void* gate_up, void* out, int rows, int inter, int64_t in_stride, int64_t out_stride,
+                      void* stream);
 
 /* out[r] = index of the first maximum of logits[r, :vocab] (mx.argmax). */
 int b200_argmax(const void* logits, int32_t* out, int rows, int vocab,

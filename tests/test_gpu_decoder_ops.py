@@ -258,3 +258,40 @@ def test_patched_model_wrapper_matches_direct_sdpa_forward():
             assert torch.equal(rt.kv_cache.key_caches[i], ref.kv_cache.key_caches[i])
     finally:
         ctx_mod.clear_context()
+
+
+@pytest.mark.parametrize("t,hq,hk,d,qk_norm,dtype", [(1100, 5, 2, 128, True, "bfloat16"), (1024, 2, 1, 64, False, "float16"),
+                                                     (3, 3, 1, 256, True, "float16"), (2, 9, 8, 256, False, "bfloat16")])
+def test_fused_norm_rope_cache_of_whole_heads(ops, t, hq, hk, d, qk_norm, dtype):
+    """The kernel for heads of 64, 128 and 256 that turn whole, where each warp has one head and where it has several, bit for
+    bit as the sequence; a value row that starts off 16 bytes; padding rows."""
+    tdt = TORCH_DT[dtype]
+    g = torch.Generator().manual_seed(t + d)
+    nb = t // 16 + 2
+    buf = torch.randn((t, (hq + 2 * hk) * d + 1), generator=g).to(tdt).cuda()[:, 1:]
+    q, k, v = (x.unflatten(1, (-1, d)) for x in buf.split([hq * d, hk * d, hk * d], dim=-1))
+    w = [(1.0 + 0.1 * torch.randn(d, generator=g)).to(tdt).cuda() if qk_norm else None for _ in range(2)]
+    pos = torch.randint(0, 9000, (t,), generator=g).int().cuda()
+    slots = torch.randperm(nb * 16, generator=g)[:t].long()
+    slots[t // 2] = -1
+    slots = slots.cuda()
+    kc, vc = (torch.randn((nb, 16, hk, d), generator=g).to(tdt).cuda() for _ in range(2))
+    q1, k1, v1, kc1, vc1 = (x.clone().contiguous() for x in (q, k, v, kc, vc))
+    if qk_norm:
+        q1, k1 = ops.rms_norm(q1, w[0], 1e-6), ops.rms_norm(k1, w[1], 1e-6)
+    ops.rope(q1, k1, pos, d, 1e6, False)
+    ops.reshape_and_cache(k1, v1, kc1, vc1, slots)
+    ops.norm_rope_cache(q, k, v, kc, vc, slots, positions=pos, rot_dim=d, base=1e6, traditional=False, q_norm_weight=w[0],
+                        k_norm_weight=w[1], eps=1e-6)
+    for name, a, b in (("q", q1, q), ("k", k1, k), ("key_cache", kc1, kc), ("value_cache", vc1, vc)):
+        assert torch.equal(a, b), name
+
+
+def test_silu_mul_as_the_next_products_operand(ops):
+    """fp16 results are the bf16 ones, saturated; rows that cannot be read in 16-byte units too."""
+    for inter in (64, 61):
+        x = torch.randn((5, 2 * inter), device="cuda").bfloat16()
+        x[1, :3], x[1, inter:inter + 3] = 3e4, 3e4
+        want = ops.silu_mul(x).float().clamp(-65504, 65504).half()
+        got = ops.silu_mul(x, out_f16=True)
+        assert got.dtype == torch.float16 and torch.equal(got, want)

@@ -159,6 +159,7 @@ EXPORTED_SYMBOLS = (
     "b200_rope",
     "b200_norm_rope_cache",
     "b200_silu_mul",
+    "b200_silu_mul_f16",
     "b200_argmax",
     "b200_add_inplace",
     "b200_advance_decode",
@@ -280,6 +281,7 @@ def load_library() -> ctypes.CDLL:
     lib.b200_norm_rope_cache.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32,
                                          f32, i64, i64, i64, i32, i64, i64, i64, i32, i64, i64, i32, vp]
     lib.b200_silu_mul.argtypes = [vp, vp, i32, i32, i64, i64, i32, vp]
+    lib.b200_silu_mul_f16.argtypes = [vp, vp, i32, i32, i64, i64, vp]
     lib.b200_argmax.argtypes = [vp, vp, i32, i32, i64, i32, vp]
     lib.b200_add_inplace.argtypes = [vp, vp, i32, i32, i64, i64, i32, vp]
     lib.b200_advance_decode.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, i32, vp]
@@ -954,10 +956,17 @@ class _Ops(HybridOps):
         self.launches += 1
         return key_cache, value_cache
 
-    def silu_mul(self, gate_up, out=None):
+    def silu_mul(self, gate_up, out=None, out_f16: bool = False):
+        """``out_f16``: a bf16 ``gate_up``'s (bf16-rounded) result as fp16, for a following quantized linear."""
         _require_cuda("gate_up", gate_up)
         inter = gate_up.shape[-1] // 2
         g2 = gate_up.reshape(-1, 2 * inter)
+        if out_f16 and out is None and gate_up.dtype == torch.bfloat16:
+            out = torch.empty((g2.shape[0], inter), dtype=torch.float16, device=gate_up.device)
+            self._check(self._lib.b200_silu_mul_f16(g2.data_ptr(), out.data_ptr(), g2.shape[0], inter, g2.stride(0),
+                                                    out.stride(0), _stream()))
+            self.launches += 1
+            return out
         if out is None:
             out = torch.empty((g2.shape[0], inter), dtype=gate_up.dtype, device=gate_up.device)
         rc = self._lib.b200_silu_mul(g2.data_ptr(), out.data_ptr(), g2.shape[0], inter, g2.stride(0),

@@ -160,7 +160,7 @@ class QuantizedLinear(nn.Module):
             y = get_ops().quantized_matmul(x, tc, self.scales, self.biases, transpose=True, group_size=self.group_size,
                                            bits=self.bits, bias=self.bias, prepacked=True)
             if self.swiglu:  # the blob's fused epilogue, unfused here
-                y = get_ops().silu_mul(y)
+                y = get_ops().silu_mul(y, out_f16=out_f16)
             return y
         if blob is not None and x.dtype in (torch.bfloat16, torch.float16):
             dt = self.scales.dtype
