@@ -182,8 +182,9 @@ norm_rope_cache_rows_kernel(T* q, T* k, const T* v, const T* __restrict__ q_norm
 #pragma unroll
     for (int j = 0; j < HALF; ++j) {
       const float a = y[j], b = y[j + HALF];
-      o[j] = from_float<T>(a * cs[j] - b * sn[j]);
-      o[j + HALF] = from_float<T>(b * cs[j] + a * sn[j]);
+      // which product the compiler fuses into the sum would be its choice: as in the general kernel
+      o[j] = from_float<T>(fmaf(a, cs[j], -__fmul_rn(b, sn[j])));
+      o[j + HALF] = from_float<T>(fmaf(b, cs[j], __fmul_rn(a, sn[j])));
     }
 #pragma unroll
     for (int j = 0; j < EPL; ++j) base[32 * j] = o[j];
