@@ -50,6 +50,9 @@ int decode_mma_ctas_per_sm(const b200_paged_attn_args& a) {
 
 template <typename T, int D, int STAGES>
 static int launch_one(const DecodeParams& p, dim3 grid, cudaStream_t st) {
+  if (p.cluster > 0)
+    return p.win_rows > 1 ? launch_decode_form<T, D, D, STAGES, true, false, false, false, true>(p, grid, st)
+                          : launch_decode_form<T, D, D, STAGES, false, false, false, false, true>(p, grid, st);
   if (p.win_rows > 1) return launch_decode_form<T, D, D, STAGES, true, false>(p, grid, st);
   return launch_decode_form<T, D, D, STAGES, false, false>(p, grid, st);
 }

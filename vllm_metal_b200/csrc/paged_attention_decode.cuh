@@ -156,7 +156,7 @@ constexpr int decode_wide_stages(int dk, int dv) {
   return fit < 2 ? 2 : fit > 4 ? 4 : fit;
 }
 
-template <typename T, int DK, int DV, int STAGES, bool WIN, bool WIDE, bool PACK, bool KEEP>
+template <typename T, int DK, int DV, int STAGES, bool WIN, bool WIDE, bool PACK, bool KEEP, bool CLUSTER>
 __global__ void __launch_bounds__(kDecodeWarps * 32, decode_ctas_per_sm(DK, DV))
 paged_decode_mma_kernel(const DecodeParams p) {
   pdl_trigger();
@@ -241,7 +241,7 @@ paged_decode_mma_kernel(const DecodeParams p) {
       ulo = max(ulo, lo);
       uhi = min(uhi, hi);
     }
-    if (!live && (WIDE || p.cluster == 0)) return;  // of a cluster it stays, with nothing to add
+    if (!live && !CLUSTER) return;  // of a cluster it stays, with nothing to add
     beg = umax > umin ? umin : 0;
     end = umax > umin ? umax : 0;
   }
@@ -531,56 +531,56 @@ paged_decode_mma_kernel(const DecodeParams p) {
   }
   __syncthreads();
 
-  if constexpr (!WIDE) {
-    if (p.cluster > 0) {
-      // the CTA's share of every row into the second half of the first warp's ring, then each CTA finishes its part of the rows
-      static_assert(STAGES * STAGE_BYTES >= 2 * 16 * DV * 4, "merged rows go beside the first warp's");
-      __shared__ float sm_cm[16], sm_cl[16];
-      float* merged = reinterpret_cast<float*>(smem_raw) + 16 * DV;
-      const int n = nrows * G * DV;
-      for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
-        const int row = idx / DV, d = idx - row * DV;
-        float M = -INFINITY, L = 0.f, acc = 0.f;
+  if constexpr (CLUSTER) {
+    // the CTA's share of every row into the second half of the first warp's ring, then each CTA finishes its part of the
+    // rows, in the order and with the roundings of split_reduce_kernel
+    static_assert(STAGES * STAGE_BYTES >= 2 * 16 * DV * 4, "merged rows go beside the first warp's");
+    __shared__ float sm_cm[16], sm_cl[16];
+    float* merged = reinterpret_cast<float*>(smem_raw) + 16 * DV;
+    const int n = nrows * G * DV;
+    for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
+      const int row = idx / DV, d = idx - row * DV;
+      float M = -INFINITY, L = 0.f, acc = 0.f;
 #pragma unroll
-        for (int w = 0; w < kDecodeWarps; ++w) M = fmaxf(M, sm_m[w][row]);
+      for (int w = 0; w < kDecodeWarps; ++w) M = fmaxf(M, sm_m[w][row]);
 #pragma unroll
-        for (int w = 0; w < kDecodeWarps; ++w) {
-          const float mw = sm_m[w][row];
-          if (mw != -INFINITY) {
-            const float wgt = exp2f(mw - M);
-            L += sm_l[w][row] * wgt;
-            acc += reinterpret_cast<const float*>(smem_raw + w * (STAGES * STAGE_BYTES))[row * DV + d] * wgt;
-          }
+      for (int w = 0; w < kDecodeWarps; ++w) {
+        const float mw = sm_m[w][row];
+        if (mw != -INFINITY) {
+          const float wgt = exp2f(mw - M);
+          L += sm_l[w][row] * wgt;
+          acc += reinterpret_cast<const float*>(smem_raw + w * (STAGES * STAGE_BYTES))[row * DV + d] * wgt;
         }
-        merged[idx] = acc;
-        if (d == 0) sm_cm[row] = M, sm_cl[row] = L;
       }
-      cluster_meet();
-      for (int idx = part * blockDim.x + threadIdx.x; idx < n; idx += p.cluster * blockDim.x) {
-        const int row = idx / DV, d = idx - row * DV, qi = WIN ? row / G : 0;
-        if (WIN && eff0 + qi <= 0) continue;
-        const int h = kvh * G + (row - qi * G);
-        float M = -INFINITY;
-        for (int j = 0; j < p.cluster; ++j) M = fmaxf(M, ld_peer(&sm_cm[row], j));
-        const float sk = p.sinks != nullptr ? p.sinks[h] * kLog2e : 0.f;
-        if (p.sinks != nullptr) M = fmaxf(M, sk);
-        if (M == -INFINITY) M = 0.f;
-        float L = 0.f, acc = 0.f;
-        for (int j = 0; j < p.cluster; ++j) {
-          const float mj = ld_peer(&sm_cm[row], j);
-          if (mj != -INFINITY) {
-            const float wgt = exp2f(mj - M);
-            L += ld_peer(&sm_cl[row], j) * wgt;
-            acc += ld_peer(&merged[idx], j) * wgt;
-          }
-        }
-        if (p.sinks != nullptr) L += exp2f(sk - M);
-        T* op = reinterpret_cast<T*>(p.out) + (int64_t)(t0 + qi) * p.out_stride + (int64_t)h * DV;
-        store_out<T>(op, d, acc / (L + p.ws.denom_eps), p.ws.out_f16);
-      }
-      cluster_meet();  // nobody leaves while a peer reads its memory
-      return;
+      merged[idx] = acc;
+      if (d == 0) sm_cm[row] = M, sm_cl[row] = L;
     }
+    cluster_meet();
+    for (int idx = part * blockDim.x + threadIdx.x; idx < n; idx += p.cluster * blockDim.x) {
+      const int row = idx / DV, d = idx - row * DV, qi = WIN ? row / G : 0;
+      if (WIN && eff0 + qi <= 0) continue;
+      const int h = kvh * G + (row - qi * G);
+      float M = -INFINITY;
+      for (int j = 0; j < p.cluster; ++j) M = fmaxf(M, ld_peer(&sm_cm[row], j));
+      const float sk = p.sinks != nullptr ? p.sinks[h] * kLog2e : 0.f;
+      if (p.sinks != nullptr) M = fmaxf(M, sk);
+      if (M == -INFINITY) M = 0.f;
+      float L = 0.f, acc = 0.f;
+      for (int j = 0; j < p.cluster; ++j) {
+        const float mj = ld_peer(&sm_cm[row], j);
+        if (mj != -INFINITY) {
+          const float wgt = exp2f(mj - M);
+          L += ld_peer(&sm_cl[row], j) * wgt;
+          acc += ld_peer(&merged[idx], j) * wgt;
+        }
+      }
+      if (p.sinks != nullptr) L += exp2f(sk - M);
+      T* op = reinterpret_cast<T*>(p.out) + (int64_t)(t0 + qi) * p.out_stride + (int64_t)h * DV;
+      const float inv = 1.f / (L + p.ws.denom_eps);
+      store_out<T>(op, d, acc * inv, p.ws.out_f16);
+    }
+    cluster_meet();  // nobody leaves while a peer reads its memory
+    return;
   }
   for (int idx = threadIdx.x; idx < nrows * G * dv; idx += blockDim.x) {
     const int row = idx / dv, d = idx - row * dv;  // MMA row = query row * G + head within the group
@@ -625,18 +625,18 @@ paged_decode_mma_kernel(const DecodeParams p) {
   }
 }
 
-template <typename T, int DK, int DV, int STAGES, bool WIN, bool WIDE, bool PACK = false, bool KEEP = false>
+template <typename T, int DK, int DV, int STAGES, bool WIN, bool WIDE, bool PACK = false, bool KEEP = false, bool CLUSTER = false>
 int launch_decode_form(const DecodeParams& p, dim3 grid, cudaStream_t st) {
   constexpr int smem = kDecodeWarps * STAGES * decode_tile_bytes(DK, DV);
+  auto kern = paged_decode_mma_kernel<T, DK, DV, STAGES, WIN, WIDE, PACK, KEEP, CLUSTER>;
   static bool configured_dev[16] = {false};  // cudaFuncSetAttribute is per device
   int dev = 0;
   B200_CUDA_OK(cudaGetDevice(&dev));
   if (!configured_dev[dev & 15]) {
-    B200_CUDA_OK(cudaFuncSetAttribute(paged_decode_mma_kernel<T, DK, DV, STAGES, WIN, WIDE, PACK, KEEP>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     configured_dev[dev & 15] = true;
   }
-  if (!WIDE && p.cluster > 0) {
+  if constexpr (CLUSTER) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kDecodeWarps * 32);
@@ -650,10 +650,10 @@ int launch_decode_form(const DecodeParams& p, dim3 grid, cudaStream_t st) {
     attr[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    B200_CUDA_OK(cudaLaunchKernelEx(&cfg, paged_decode_mma_kernel<T, DK, DV, STAGES, WIN, WIDE, PACK, KEEP>, p));
-    return B200_OK;
+    B200_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, p));
+    return check_launch("paged_decode_mma_kernel (cluster)");
   }
-  launch_pdl(paged_decode_mma_kernel<T, DK, DV, STAGES, WIN, WIDE, PACK, KEEP>, grid, dim3(kDecodeWarps * 32), smem, st, p);
+  launch_pdl(kern, grid, dim3(kDecodeWarps * 32), smem, st, p);
   return check_launch("paged_decode_mma_kernel");
 }
 

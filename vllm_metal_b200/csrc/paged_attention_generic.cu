@@ -277,8 +277,6 @@ static int effective_span(const b200_paged_attn_args& a) {
   return L < 1 ? 1 : L;
 }
 
-constexpr int kClusterPartition = 1024;  // tokens; longer rows take more partitions than a cluster has CTAs
-
 // Returns the partition length in tokens (a multiple of b200_partition_size())
 // and the partition count through *parts; parts == 1 means single pass.
 static int plan_partitions(const b200_paged_attn_args& a, bool mma, int* parts, int* cluster) {
@@ -287,21 +285,6 @@ static int plan_partitions(const b200_paged_attn_args& a, bool mma, int* parts, 
   const int span = effective_span(a);
   const int max_parts = (span + unit - 1) / unit;  // paged_ops.cpp:520-521
   *parts = 1;
-  // Few rows: short partitions in the CTAs of one cluster, merged through its shared memory -- the chip has idle SMs and a row's
-  // time is its tiles one after another.  All clusters at once only: past that the longer partitions below share the chip better.
-  // One row of 8 kv heads at 512 tokens (planned for 1024): 16 CTAs and a merge launch 13.9 us, 64 CTAs in clusters 7.2.
-  if (mma && a.force_partitions == 0 && decode_cluster_supported(a)) {
-    const int sms = sm_count() > 0 ? sm_count() : 148;
-    const int64_t items = (int64_t)a.num_kv_heads * a.num_q_tokens;
-    int np = 8;
-    while (np > 1 && (items * np > sms || (span + np - 1) / np < 64)) np /= 2;
-    const int psz = (((span + np - 1) / np + 63) / 64) * 64;
-    if (np > 1 && psz <= kClusterPartition) {
-      *cluster = np;
-      *parts = 1;
-      return psz;
-    }
-  }
   if (a.force_partitions == 1 || max_parts < 2) return unit;
   if (a.force_partitions > 1) {
     *parts = max_parts;
@@ -334,6 +317,13 @@ static int plan_partitions(const b200_paged_attn_args& a, bool mma, int* parts, 
           best_p = np;
           best_size = psz;
         }
+      }
+      // All CTAs resident at once and few partitions a row: its CTAs form a cluster and merge through each other's shared memory,
+      // with the same results -- no scratch, no merge launch.  With more CTAs than that a cluster's early ones would hold their
+      // places while the others work.  One row of 8 kv heads at 512 tokens (planned for 1024): 13.9 -> 11.86 us.
+      if (best_p > 1 && best_p <= 8 && items * best_p <= slots && decode_cluster_supported(a)) {
+        *cluster = best_p;
+        return best_size;
       }
       *parts = best_p;
       return best_size;
