@@ -105,7 +105,7 @@ class PagedModelRunner:
         self.block_size = kv_cache.block_size
         self.max_batch = max_batch
         self.max_blocks = (max_model_len + self.block_size - 1) // self.block_size
-        # the MoE expert path reads its per-expert row counts back to the host every block: not capturable
+        # blocks of sizes that the grouped expert kernels do not take read row counts back to the host: not capturable
         has_moe = any(hasattr(getattr(layer, "mlp", None), "block") for layer in getattr(model, "layers", []))
         self.use_cuda_graph = use_cuda_graph and not has_moe
         # recurrent layers: every request owns a state slot, named by the caller step for step
