@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
     (16, 8, 128, [513], 1, -1, False, 1024),          # one token of the second partition
     (16, 8, 64, [1], 1, -1, True, 1536),              # one token: all but one CTA have nothing; a cluster of 3
     (4, 1, 128, [700, 3, 4000], 1, -1, True, 4096),   # a cluster of 8
-    (8, 2, 64, [100, 2000], 1, 700, False, 2048),     # a window shorter than the plan
+    (8, 2, 64, [100, 2000], 1, 1500, False, 2048),    # a window shorter than the plan: 3 partitions of 512 (700 would be one of 704)
     (8, 2, 128, [1700, 65], 1, 1000, True, 2048),
     (8, 1, 64, [300, 17, 1000], 3, -1, False, 1024),  # verification windows, rows that end before a partition
     (32, 2, 128, [1029], 2, 1000, True, 1536),
