@@ -295,3 +295,28 @@ def test_silu_mul_as_the_next_products_operand(ops):
         want = ops.silu_mul(x).float().clamp(-65504, 65504).half()
         got = ops.silu_mul(x, out_f16=True)
         assert got.dtype == torch.float16 and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+def test_norm_weights_that_the_launch_before_makes(ops, d):
+    """The fused kernel starts while the launch before it works: it reads the norms' weights after the wait for it."""
+    g = torch.Generator(device="cuda").manual_seed(d)
+    t, hq, hk, nb = 64, 8, 2, 5
+    made = torch.ones((8192, 4096), dtype=torch.bfloat16, device="cuda")  # the weights are its last row's ends: written last
+    delta = torch.full_like(made, 0.5)
+    pos = torch.arange(t, dtype=torch.int32, device="cuda")
+    slots = torch.arange(t, dtype=torch.int64, device="cuda")
+    qkv = torch.randn((t, hq + 2 * hk, d), device="cuda", generator=g).bfloat16()
+    outs = []
+    for early in (True, False):
+        made.fill_(1.0)
+        q, k, v = (x.contiguous() for x in qkv.split([hq, hk, hk], dim=1))
+        kc, vc = (torch.zeros((nb, 16, hk, d), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        ops.add_(made, delta)
+        if not early:
+            torch.cuda.synchronize()
+        ops.norm_rope_cache(q, k, v, kc, vc, slots, positions=pos, rot_dim=d, base=1e6, q_norm_weight=made[-1, :d],
+                            k_norm_weight=made[-1, -d:], eps=1e-6)
+        outs.append((q, k, kc, vc))
+    for a, b in zip(*outs, strict=True):
+        assert torch.equal(a, b)

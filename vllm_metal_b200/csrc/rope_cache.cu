@@ -120,7 +120,7 @@ norm_rope_cache_kernel(T* __restrict__ q, T* __restrict__ k, const T* __restrict
 // heads, with norms 69 -> 26 us, without 56 -> 20.
 template <typename T, int EPL>
 __global__ void __launch_bounds__(RC_WARPS * 32)
-norm_rope_cache_rows_kernel(T* q, T* k, const T* v, const T* __restrict__ q_norm_w, const T* __restrict__ k_norm_w,
+norm_rope_cache_rows_kernel(T* q, T* k, const T* v, const T* q_norm_w, const T* k_norm_w,
                             const int32_t* positions, const int64_t* slot_mapping, T* key_cache, T* value_cache, int num_q_heads,
                             int num_kv_heads, float log2_base, float eps, int64_t q_stride, int64_t k_stride, int64_t v_stride,
                             int block_size, int64_t num_slots, int64_t kv_block_stride, int64_t kv_token_stride, int value_dim,
@@ -128,15 +128,9 @@ norm_rope_cache_rows_kernel(T* q, T* k, const T* v, const T* __restrict__ q_norm
   constexpr int D = 32 * EPL, HALF = EPL / 2;
   const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_trigger();
-  // nothing here was written by an earlier launch
-  float inv_freq[HALF], qw[EPL], kw[EPL];
+  float inv_freq[HALF];  // of arguments alone: every operand, the norms' weights too, may be an earlier launch's result
 #pragma unroll
   for (int j = 0; j < HALF; ++j) inv_freq[j] = exp2f(-log2_base * (2.f * (float)(lane + 32 * j) / (float)D));
-#pragma unroll
-  for (int j = 0; j < EPL; ++j) {
-    qw[j] = q_norm_w ? to_float(q_norm_w[lane + 32 * j]) : 0.f;
-    kw[j] = k_norm_w ? to_float(k_norm_w[lane + 32 * j]) : 0.f;
-  }
   pdl_wait();
   const int heads = num_q_heads + num_kv_heads, step = RC_WARPS * gridDim.y;
   T* qt = q + (int64_t)t * q_stride + lane;
@@ -148,6 +142,12 @@ norm_rope_cache_rows_kernel(T* q, T* k, const T* v, const T* __restrict__ q_norm
     const T* p = head_at(h);
 #pragma unroll
     for (int j = 0; j < EPL; ++j) x[j] = p[32 * j];
+  }
+  T qw[EPL], kw[EPL];
+#pragma unroll
+  for (int j = 0; j < EPL; ++j) {
+    qw[j] = q_norm_w ? q_norm_w[lane + 32 * j] : from_float<T>(0.f);
+    kw[j] = k_norm_w ? k_norm_w[lane + 32 * j] : from_float<T>(0.f);
   }
   const float pos = (float)positions[t];
   const int64_t slot = slot_mapping[t];
@@ -176,7 +176,7 @@ norm_rope_cache_rows_kernel(T* q, T* k, const T* v, const T* __restrict__ q_norm
       ss = warp_sum(ss);
       const float inv = rsqrtf(ss / (float)D + eps);
 #pragma unroll
-      for (int j = 0; j < EPL; ++j) y[j] = to_float(from_float<T>(y[j] * inv * (is_q ? qw[j] : kw[j])));
+      for (int j = 0; j < EPL; ++j) y[j] = to_float(from_float<T>(y[j] * inv * to_float(is_q ? qw[j] : kw[j])));
     }
     T o[EPL];
 #pragma unroll
