@@ -108,3 +108,83 @@ def test_the_parts_and_the_whole_agree(top, tokens):
     parts = blk.experts(x, idx)
     want = (parts.float() * scores[..., None]).sum(1)
     torch.testing.assert_close(y.float(), want, rtol=2**-7, atol=1e-5)
+
+
+def _by_parts(blk, x, idx, scores):
+    """The block's result for choices that are given, each expert's GEMM by itself."""
+    from vllm_metal_b200.quant import switch_linear as sl
+
+    glu = blk.experts
+    order, counts = sl._sort_pairs(idx, glu.gate_proj.num_experts)
+    xs = sl._f16_operand(x.index_select(0, order // idx.shape[1]).contiguous(), glu.gate_proj)
+    g, u = (sl.QuantizedSwitchLinear.forward_sorted(m, xs, counts) for m in (glu.gate_proj, glu.up_proj))
+    h = sl.ACTIVATIONS[glu.activation](g.float(), u.float()).to(g.dtype)
+    ys = sl.QuantizedSwitchLinear.forward_sorted(glu.down_proj, sl._f16_operand(h, glu.down_proj), counts)
+    out = torch.empty_like(ys)
+    out[order] = ys
+    return (out.unflatten(0, idx.shape).float() * scores[..., None]).sum(1)
+
+
+@pytest.mark.parametrize("how", ["subclass", "instance", "class"])
+def test_a_route_of_ones_own_is_asked(how, monkeypatch):
+    blk = _block(128, 64, 7, 2, 4, 64, "silu", "topk_softmax", False)
+    x = torch.randn((9, 128), device="cuda").bfloat16()
+
+    def route(self, x):
+        idx = torch.tensor([[6, 0]], device=x.device).expand(x.shape[0], 2)
+        return idx, torch.full(idx.shape, 0.5, device=x.device)
+
+    if how == "subclass":
+        blk.__class__ = type("Own", (type(blk),), {"route": route})
+    elif how == "instance":
+        blk.route = route.__get__(blk)
+    else:
+        monkeypatch.setattr(type(blk), "route", route)
+    want = _by_parts(blk, x, *route(blk, x))
+    torch.testing.assert_close(blk(x).float(), want, rtol=2**-7, atol=1e-3)
+
+
+@pytest.mark.parametrize("where", ["router", "experts"])
+def test_hooks_and_forwards_of_ones_own_run(where):
+    blk = _block(128, 64, 7, 2, 4, 64, "silu", "softmax_topk", False)
+    x = torch.randn((9, 128), device="cuda").bfloat16()
+    plain = blk(x)
+    m = getattr(blk, where)
+    seen = []
+    for add in (m.register_forward_hook, m.register_forward_pre_hook):
+        handle = add(lambda *a: seen.append(1))
+        torch.testing.assert_close(blk(x).float(), plain.float(), rtol=2**-7, atol=1e-3)
+        handle.remove()
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda mod, a, out: seen.append(1) if mod is m else None)
+    blk(x)
+    handle.remove()
+    assert len(seen) == 3
+    m.forward = lambda *a: type(m).forward(m, *a) * 0
+    y = blk(x)
+    assert (y == 0).all() if where == "experts" else not torch.equal(y, plain)
+
+
+@pytest.mark.parametrize("which", ["gate_proj", "up_proj", "down_proj"])
+def test_a_projection_of_ones_own_is_asked(which):
+    blk = _block(128, 64, 7, 2, 4, 64, "silu", "topk_softmax", False)
+    x = torch.randn((9, 128), device="cuda").bfloat16()
+    m = getattr(blk.experts, which)
+    m.__class__ = type("Own", (type(m),), {"forward_sorted": lambda self, xs, counts: super(type(self), self).forward_sorted(xs, counts) * 0})
+    assert (blk(x) == 0).all() and (blk.experts(x, blk.route(x)[0]) == 0).all()
+
+
+def test_routers_that_are_no_buffers_of_a_router():
+    """A weight that is a Parameter, with gradients through the scores as before; a plain function."""
+    blk = _block(128, 64, 7, 2, 4, 64, "silu", "topk_softmax", False)
+    x = torch.randn((9, 128), device="cuda").bfloat16()
+    plain, w = blk(x), blk.router.weight
+    del blk.router.weight
+    blk.router.weight = torch.nn.Parameter(w)
+    y = blk(x)
+    y.float().square().sum().backward()
+    assert blk.router.weight.grad.abs().sum() > 0
+    with torch.no_grad():
+        assert torch.equal(blk(x), plain)
+    del blk.router
+    blk.router = lambda z: z @ w.t()
+    torch.testing.assert_close(blk(x), plain, rtol=2**-6, atol=2e-3)

@@ -261,3 +261,43 @@ def test_switch_linear_shards_are_slices_of_the_stacked_experts():
         np.testing.assert_allclose(part, full, rtol=1e-10, atol=1e-10)
     with pytest.raises(ValueError):
         sw.shard_cols(0, 8)  # 256 / 8 = 32 is not a multiple of the group size
+
+
+def test_expert_block_with_a_router_that_is_a_function():
+    """A router need not be a module; experts of any kind are called with the rows and the choices."""
+    import torch
+
+    from vllm_metal_b200.quant.switch_linear import MoEBlock
+
+    w = torch.randn((5, 8), generator=torch.Generator().manual_seed(0))
+    blk = MoEBlock(lambda x: x @ w.t(), lambda x, idx: x[:, None, :] * (idx[..., None] + 1), 2)
+    x = torch.randn((3, 8), generator=torch.Generator().manual_seed(1))
+    idx, scores = blk.route(x)
+    torch.testing.assert_close(blk(x), (x[:, None] * (idx[..., None] + 1) * scores[..., None]).sum(1))
+
+
+def test_what_the_grouped_expert_kernels_may_stand_for():
+    import torch
+
+    from vllm_metal_b200.quant import switch_linear as sl
+
+    r = sl.Router(8, 4, False)
+    assert sl._as_defined(r, sl.Router, "forward")
+    for m in (type("Own", (sl.Router,), {})(8, 4, False), torch.nn.Linear(8, 4), lambda x: x):
+        assert not sl._as_defined(m, sl.Router, "forward")
+    for add in (r.register_forward_hook, r.register_forward_pre_hook, r.register_full_backward_hook):
+        handle = add(lambda *a: None)
+        assert not sl._as_defined(r, sl.Router, "forward")
+        handle.remove()
+    handle = torch.nn.modules.module.register_module_forward_pre_hook(lambda *a: None)
+    assert not sl._as_defined(r, sl.Router, "forward")
+    handle.remove()
+    assert sl._as_defined(r, sl.Router, "forward")
+    r.forward = lambda x: x
+    assert not sl._as_defined(r, sl.Router, "forward")
+    x = torch.ones(2)
+    assert not sl._differentiated(x, None) and sl._differentiated(x, torch.ones(2, requires_grad=True))
+    with torch.no_grad():
+        assert not sl._differentiated(torch.ones(2, requires_grad=True))
+    with torch.autograd.forward_ad.dual_level():
+        assert sl._differentiated(x)

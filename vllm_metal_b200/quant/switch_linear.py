@@ -20,6 +20,8 @@ from __future__ import annotations
 
 import torch
 from torch import nn
+from torch.autograd import forward_ad
+from torch.nn.modules.module import _has_any_global_hook as _any_global_hook
 
 from ..metal import get_ops
 from .affine import quantize
@@ -152,6 +154,19 @@ _GROUPED_ACTIVATIONS = {"silu": (_act_silu, 0), "gpt_oss": (_act_gpt_oss, 1)}  #
 _WORDS = (torch.int32, torch.uint32)
 
 
+def _as_defined(m, cls: type, *methods: str) -> bool:
+    """Whether a call of ``m`` runs nothing but ``cls``'s methods as they stand in their module: no class of its own, no method
+    replaced on the instance or the class, no hooks.  The grouped kernels take the place of such modules only."""
+    return (type(m) is cls and all(getattr(cls, n) is _DEFINED[cls][n] and n not in m.__dict__ for n in methods)
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+            and not _any_global_hook())
+
+
+def _differentiated(*tensors) -> bool:
+    """Whether a derivative is being taken that reaches one of these: the grouped kernels leave no trace of theirs."""
+    return forward_ad._current_level >= 0 or (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors))
+
+
 class SwitchGLU(nn.Module):
     """``down(act(gate(x), up(x)))`` per selected expert (mlx-lm ``SwitchGLU``).  The activation runs in fp32 on the
     dtype-rounded projections and is rounded once."""
@@ -165,11 +180,12 @@ class SwitchGLU(nn.Module):
 
     def grouped_tile_rows(self, x: torch.Tensor, top: int) -> int:
         """Rows per tile with which the grouped kernels take ``x [T, H]``, 0 if they do not.  They take bf16 rows and affine
-        parameters, widths that are multiples of 64 and 16-byte aligned tensors; gradients pass through the other path."""
+        parameters, widths that are multiples of 64 and 16-byte aligned tensors, of projections that are nothing but a
+        ``QuantizedSwitchLinear``; gradients pass through the other path."""
         g, u, d = self.gate_proj, self.up_proj, self.down_proj
         if (x.dtype != torch.bfloat16 or not x.is_cuda or x.shape[0] == 0 or self.activation not in _GROUPED_ACTIVATIONS
-                or ACTIVATIONS[self.activation] is not _GROUPED_ACTIVATIONS[self.activation][0]
-                or (torch.is_grad_enabled() and x.requires_grad)):
+                or ACTIVATIONS[self.activation] is not _GROUPED_ACTIVATIONS[self.activation][0] or _differentiated(x)
+                or not all(_as_defined(m, QuantizedSwitchLinear, "forward_sorted") for m in (g, u, d))):
             return 0
         ops = get_ops()
         if getattr(ops, "_qlinear_kernel", 0) == 1 or (g.bits, g.group_size) != (u.bits, u.group_size):
@@ -261,37 +277,36 @@ class MoEBlock(nn.Module):
     def _choose(self, x: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor] | None:
         """Router product and choice in one launch, ``(int32, fp32)`` of ``[T, k]``; ``None`` where it does not apply."""
         r = self.router
-        if (type(r) is not Router or not x.is_cuda or x.dtype != torch.bfloat16 or x.shape[0] == 0
-                or (torch.is_grad_enabled() and x.requires_grad)):
+        if not x.is_cuda or x.dtype != torch.bfloat16 or x.shape[0] == 0 or not _as_defined(r, Router, "forward"):
             return None
         w, b = r.weight, r.bias
-        if (x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16 or x.shape[1] % 32 or w.shape[1] != x.shape[1] or w.dtype != x.dtype
-                or not w.is_contiguous() or w.data_ptr() % 16 or w.device != x.device or w.shape[0] > 128
+        if (_differentiated(x, w, b) or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16 or x.shape[1] % 32
+                or w.shape[1] != x.shape[1] or w.dtype != x.dtype or not w.is_contiguous() or w.data_ptr() % 16 or w.device != x.device or w.shape[0] > 128
                 or not 1 <= self.top_k <= min(32, w.shape[0])
                 or (b is not None and (b.dtype != x.dtype or not b.is_contiguous() or b.device != x.device))):
             return None
         return get_ops().qexpert_route(x, w, b, self.top_k, self.routing == "softmax_topk", self.norm_topk_prob)
 
     def _whole(self, x: torch.Tensor) -> torch.Tensor | None:
-        """The block in one call, ``None`` where that does not apply (what is checked here: types, shapes and strides; sizes and
-        alignment by the call)."""
-        r, glu = self._modules["router"], self._modules["experts"]
-        act = _GROUPED_ACTIVATIONS.get(getattr(glu, "activation", None))
-        if (type(r) is not Router or type(glu) is not SwitchGLU or self.trace is not None or x.dtype != torch.bfloat16 or not x.is_cuda
-                or act is None or ACTIVATIONS[glu.activation] is not act[0] or x.shape[0] == 0 or x.stride(1) != 1
-                or (x.requires_grad and torch.is_grad_enabled())):
+        """The block in one call, ``None`` where that does not apply (what is checked here: code that a call would run beside the
+        kernels', types, shapes and strides; sizes and alignment by the call)."""
+        r, glu = self.router, self.experts
+        if (x.dtype != torch.bfloat16 or not x.is_cuda or x.shape[0] == 0 or x.stride(1) != 1 or self.trace is not None
+                or not self._routes_as_defined() or not _as_defined(r, Router, "forward") or not _as_defined(glu, SwitchGLU, "forward")):
+            return None
+        act = _GROUPED_ACTIVATIONS.get(glu.activation)
+        lins = (glu.gate_proj, glu.up_proj, glu.down_proj)
+        if act is None or ACTIVATIONS[glu.activation] is not act[0] or not all(_as_defined(m, QuantizedSwitchLinear, "forward_sorted")
+                                                                               for m in lins):
             return None
         ops, dev, h = get_ops(), x.device, x.shape[1]
-        if getattr(ops, "_qlinear_kernel", 0) == 1:
-            return None
-        lins = [glu._modules[n] for n in ("gate_proj", "up_proj", "down_proj")]
         bits, group = lins[0].bits, lins[0].group_size
-        if bits not in (4, 8) or group not in (32, 64, 128) or any(type(m) is not QuantizedSwitchLinear or m.bits != bits or m.group_size != group
-                                                                   for m in lins):
+        if (getattr(ops, "_qlinear_kernel", 0) == 1 or bits not in (4, 8) or group not in (32, 64, 128)
+                or any(m.bits != bits or m.group_size != group for m in lins)):
             return None
-        bufs = [(b["weight"], b["scales"], b["biases"], b.get("bias")) for b in (m._buffers for m in lins)]
-        e, f = bufs[0][1].shape[:2]
-        for (w, s, b, extra), n, k in zip(bufs, (f, f, h), (h, h, f), strict=True):
+        mats = [(m.weight, m.scales, m.biases, m.bias) for m in lins]
+        e, f = mats[0][1].shape[:2]
+        for (w, s, b, extra), n, k in zip(mats, (f, f, h), (h, h, f), strict=True):
             if (s.dtype is not torch.bfloat16 or b.dtype is not torch.bfloat16 or w.dtype not in _WORDS or s.shape != (e, n, k // group)
                     or b.shape != s.shape or w.shape != (e, n, k * bits // 32) or w.device != dev or s.device != dev or b.device != dev
                     or not (w.is_contiguous() and s.is_contiguous() and b.is_contiguous())):
@@ -299,11 +314,15 @@ class MoEBlock(nn.Module):
             if extra is not None and (extra.dtype is not torch.bfloat16 or extra.shape != (e, n) or extra.device != dev
                                       or not extra.is_contiguous()):
                 return None
-        rw, rb = r._buffers["weight"], r._buffers.get("bias")
+        rw, rb = r.weight, r.bias
         if (rw.dtype is not torch.bfloat16 or rw.shape != (e, h) or rw.device != dev or not rw.is_contiguous() or (rb is not None and (
-                rb.dtype is not torch.bfloat16 or rb.shape != (e,) or rb.device != dev or not rb.is_contiguous()))):
+                rb.dtype is not torch.bfloat16 or rb.shape != (e,) or rb.device != dev or not rb.is_contiguous()))
+                or _differentiated(x, rw, rb)):
             return None
-        return ops.qexpert_block(x, (rw, rb), bufs, bits, group, self.top_k, act[1], self.routing == "softmax_topk", self.norm_topk_prob)
+        return ops.qexpert_block(x, (rw, rb), mats, bits, group, self.top_k, act[1], self.routing == "softmax_topk", self.norm_topk_prob)
+
+    def _routes_as_defined(self) -> bool:
+        return type(self).route is _DEFINED[MoEBlock]["route"] and "route" not in self.__dict__
 
     def route(self, x: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
         got = self._choose(x) if x.dim() == 2 else None
@@ -328,16 +347,22 @@ class MoEBlock(nn.Module):
         y = self._whole(x2)
         if y is not None:
             return y.reshape(*lead, -1)
-        tile_rows = self.experts.grouped_tile_rows(x2, self.top_k) if isinstance(self.experts, SwitchGLU) else 0
-        got = self._choose(x2) if tile_rows else None
+        tile_rows = self.experts.grouped_tile_rows(x2, self.top_k) if _as_defined(self.experts, SwitchGLU, "forward") else 0
+        known = tile_rows and self._routes_as_defined()
+        got = self._choose(x2) if known else None
         idx, scores = got if got is not None else self.route(x2)
         if self.trace is not None:
-            self.trace.append((idx.cpu().numpy(), scores.cpu().numpy()))
-        if (tile_rows and scores.dtype == torch.float32 and not (torch.is_grad_enabled() and scores.requires_grad)
-                and type(self.router) in (Router, nn.Linear) and self.router.weight.shape[0] <= self.experts.gate_proj.num_experts):
+            self.trace.append((idx.to(torch.int64).cpu().numpy(), scores.cpu().numpy()))
+        if (known and scores.dtype == torch.float32 and not _differentiated(scores)
+                and (_as_defined(self.router, Router, "forward") or _as_defined(self.router, nn.Linear, "forward"))
+                and self.router.weight.shape[0] <= self.experts.gate_proj.num_experts):
             # no more logits than there are experts: the choices are in range
             y = self.experts.grouped(x2, idx.to(torch.int32), tile_rows)
             return get_ops().qexpert_sum(y, scores.contiguous()).reshape(*lead, -1)
         y = self.experts(x2, idx)  # [T, k, hidden]
         out = (y.float() * scores[..., None]).sum(dim=1).to(x.dtype)
         return out.reshape(*lead, -1)
+
+
+_DEFINED = {QuantizedSwitchLinear: {"forward_sorted": QuantizedSwitchLinear.forward_sorted}, SwitchGLU: {"forward": SwitchGLU.forward},
+            Router: {"forward": Router.forward}, nn.Linear: {"forward": nn.Linear.forward}, MoEBlock: {"route": MoEBlock.route}}
