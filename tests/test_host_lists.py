@@ -48,3 +48,44 @@ def test_slots_of_a_window_of_pages():
         assert _slots(ids, first, count, 16) == want == _slots(np.array(ids), first, count, 16)
     with pytest.raises(IndexError):
         _slots(ids, 630, 40, 16)
+
+
+@pytest.mark.parametrize("broken", ["compiler", "no compiler", "no source"])
+def test_the_library_builds_without_the_converter(broken, monkeypatch, tmp_path):
+    """A box with a fresh library, or with nvcc alone, needs no C compiler: lists then go through NumPy."""
+    from vllm_metal_b200.metal import build as b
+
+    lib = tmp_path / "lib.so"
+    lib.touch()
+    monkeypatch.setattr(b, "output_path", lambda component=None: lib)
+    monkeypatch.setattr(b, "stale_artifacts", lambda component=None: [])
+    monkeypatch.setattr(b, "_PKG_DIR", tmp_path)
+    if broken == "no source":
+        monkeypatch.setattr(b, "CSRC_DIR", tmp_path)
+    else:
+        monkeypatch.setenv("CC", "false" if broken == "compiler" else str(tmp_path / "cc"))
+    with pytest.warns(RuntimeWarning, match="NumPy"):
+        assert b.build() == lib
+    assert sorted(tmp_path.iterdir()) == [lib]
+
+
+def test_the_converter_is_fresh_by_content_and_named_by_interpreter(monkeypatch, tmp_path):
+    import os
+    import sysconfig
+
+    from vllm_metal_b200.metal import build as b
+
+    monkeypatch.setattr(b, "_PKG_DIR", tmp_path)
+    src = tmp_path / "csrc" / "host_lists.c"
+    src.parent.mkdir()
+    src.write_bytes((b.CSRC_DIR / "host_lists.c").read_bytes())
+    monkeypatch.setattr(b, "CSRC_DIR", src.parent)
+    out = b.build_host()
+    assert sysconfig.get_config_var("SOABI") in out.name
+    made = out.stat().st_mtime_ns
+    os.utime(src, (out.stat().st_mtime + 100,) * 2)  # a new checkout of the same source
+    assert b.build_host().stat().st_mtime_ns == made
+    src.write_text(src.read_text() + "\n/* changed */\n")
+    os.utime(src, (1, 1))
+    assert b.build_host().stat().st_mtime_ns != made
+    assert not list(tmp_path.glob(".host_*"))

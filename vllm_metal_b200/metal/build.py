@@ -15,6 +15,9 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
+import tempfile
+import warnings
 from pathlib import Path
 
 _PKG_DIR = Path(__file__).resolve().parent.parent
@@ -61,20 +64,29 @@ def output_path(component: str | None = None) -> Path:
 
 
 def host_library_path() -> Path:
-    return _PKG_DIR / "lib_b200_host.so"
+    """The list converter's library; it reads the interpreter's own structures, so its name carries that interpreter's ABI."""
+    return _PKG_DIR / f"lib_b200_host{sysconfig.get_config_var('EXT_SUFFIX') or '.so'}"
 
 
 def build_host(force: bool = False) -> Path:
-    """``csrc/host_lists.c`` with the C compiler, against this interpreter's headers."""
-    import sysconfig
-
+    """``csrc/host_lists.c`` with the C compiler, against this interpreter's headers; fresh by content, put in place whole."""
     out, src = host_library_path(), CSRC_DIR / "host_lists.c"
-    if not force and out.exists() and out.stat().st_mtime >= src.stat().st_mtime:
-        return out
-    cmd = [os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I", sysconfig.get_path("include"), "-o", str(out), str(src)]
-    proc = subprocess.run(cmd, capture_output=True, text=True)
-    if proc.returncode != 0:
-        raise RuntimeError(f"{cmd[0]} failed ({proc.returncode}) on {src.name}:\n{proc.stderr[-4000:]}")
+    stamp = out.with_name(out.name + ".stamp")
+    cmd = [os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I", sysconfig.get_path("include")]
+    try:
+        tag = hashlib.sha256(src.read_bytes()).hexdigest()
+        if not force and out.exists() and stamp.exists() and stamp.read_text().strip() == tag:
+            return out
+        with tempfile.TemporaryDirectory(dir=out.parent, prefix=".host_") as tmp:
+            made, mark = Path(tmp) / out.name, Path(tmp) / stamp.name
+            proc = subprocess.run([*cmd, "-o", str(made), str(src)], capture_output=True, text=True)
+            if proc.returncode != 0:
+                raise RuntimeError(f"{cmd[0]} failed ({proc.returncode}) on {src.name}:\n{proc.stderr[-4000:]}")
+            mark.write_text(tag + "\n")
+            os.replace(made, out)
+            os.replace(mark, stamp)
+    except OSError as e:
+        raise RuntimeError(f"{src.name} was not built: {e}") from e
     return out
 
 
@@ -142,7 +154,10 @@ def build(force: bool = False, verbose: bool = False, component: str | None = No
     from concurrent.futures import ThreadPoolExecutor
 
     out = output_path(component)
-    build_host(force)
+    try:
+        build_host(force)
+    except RuntimeError as e:  # host_lists.py does without it
+        warnings.warn(f"lists of page numbers will be converted by NumPy: {e}", RuntimeWarning, stacklevel=2)
     if not force and out.exists() and not stale_artifacts(component):
         return out
     extra = os.environ.get("B200_NVCC_EXTRA", "").split()  # tuning experiments (-DQGEMM_...), not for shipping
