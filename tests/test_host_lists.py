@@ -89,3 +89,11 @@ def test_the_converter_is_fresh_by_content_and_named_by_interpreter(monkeypatch,
     os.utime(src, (1, 1))
     assert b.build_host().stat().st_mtime_ns != made
     assert not list(tmp_path.glob(".host_*"))
+
+
+@pytest.mark.parametrize("values", [[3, -1, 2**31 - 1], [2**32 + 5, 1], np.array([2**32 + 5, -1]), [np.int64(2**32 + 5)], (7, 8), []])
+def test_slots_keep_their_64_bits(values):
+    from vllm_metal_b200.attention.impls.sdpa import _as_int64
+
+    got = _as_int64(values)
+    assert got.dtype == np.int64 and got.tolist() == [int(v) for v in values]

@@ -21,7 +21,7 @@ from ...metal import get_ops
 from ...metal.constants import KERNEL_BLOCK_SIZES
 from ..caches.kv_cache import B200PagedKVCache
 from ..context import PagedAttentionContext
-from ...host_lists import as_int32, fill_rows
+from ...host_lists import fill_rows, native_int32
 
 
 # Test knob: False runs the reference's step-by-step sequence (norm, rope, reshape_and_cache as
@@ -62,11 +62,9 @@ def _build_block_tables_np(raw_block_tables: list[list[int]], cache_block_size: 
 
 
 def _as_int64(values) -> np.ndarray:
-    """Slots fit 32 bits in all but the largest caches: converted that way first."""
-    try:
-        return as_int32(values).astype(np.int64)
-    except OverflowError:
-        return np.asarray(values, dtype=np.int64)
+    """Slots: lists of integers by way of 32 bits, which all but the largest caches' fit; anything else with all its 64."""
+    fast = native_int32(values)
+    return np.asarray(values, dtype=np.int64) if fast is None else fast.astype(np.int64)
 
 
 def _build_block_tables(raw_block_tables, cache_block_size, device="cuda"):

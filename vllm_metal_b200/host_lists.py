@@ -35,11 +35,18 @@ def fill_rows(dst: np.ndarray, rows) -> None:
         dst[i, : len(row)] = row
 
 
-def as_int32(values) -> np.ndarray:
-    """``np.asarray(values, dtype=np.int32)``."""
+def native_int32(values) -> np.ndarray | None:
+    """A list of Python integers that fit as int32; ``None`` for anything else, which the caller's general conversion then takes
+    or refuses."""
     lib = _lib()
     if lib is not None and type(values) is list and values:
         out = np.empty(len(values), dtype=np.int32)
         if lib.b200_host_fill_row(values, out.ctypes.data, len(values)) == 0:
             return out
-    return np.asarray(values, dtype=np.int32)
+    return None
+
+
+def as_int32(values) -> np.ndarray:
+    """``np.asarray(values, dtype=np.int32)``."""
+    fast = native_int32(values)
+    return np.asarray(values, dtype=np.int32) if fast is None else fast
