@@ -481,3 +481,22 @@ def test_worker_deferred_sampling_emits_the_synchronous_stream():
     sync, piped = run(False), run(True)
     assert {r: len(v) for r, v in piped.items()} == {r: len(v) for r, v in sync.items()}
     assert piped == sync
+
+
+def test_token_ids_that_are_on_the_device():
+    """A step takes a CUDA tensor of ids, or its scalars, as it takes a list."""
+    from vllm_metal_b200.attention.caches.kv_cache import B200PagedKVCache
+    from vllm_metal_b200.lm.decoder import PRESETS, Model
+    from vllm_metal_b200.v1.model_runner import PagedModelRunner
+
+    args = PRESETS["tiny"]
+    model = Model(args, torch.bfloat16, "cuda", seed=0)
+    cache = B200PagedKVCache(args.num_layers, args.n_kv_heads, args.head_dim, 4, 16, torch.bfloat16, "cuda",
+                             sliding_window_per_layer=args.sliding_window_per_layer())
+    runner = PagedModelRunner(model, cache, max_batch=1, max_model_len=32, use_cuda_graph=False)
+    ids = list(range(1, 9))
+    want = runner.execute(ids, [], [([1], 8, 0)])
+    logits = runner.last_logits.clone()
+    for form in (torch.tensor(ids, device="cuda"), list(torch.tensor(ids, device="cuda")), tuple(ids), np.array(ids)):
+        assert runner.execute(form, [], [([1], 8, 0)]) == want and torch.equal(runner.last_logits, logits)
+        assert runner.verify(form, [([1], 0, 8)])[0][-1] == want[0]

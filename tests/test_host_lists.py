@@ -97,3 +97,17 @@ def test_slots_keep_their_64_bits(values):
 
     got = _as_int64(values)
     assert got.dtype == np.int64 and got.tolist() == [int(v) for v in values]
+
+
+def test_token_ids_as_torch_takes_them():
+    import torch
+
+    from vllm_metal_b200.v1.model_runner import _token_ids
+
+    for ids in ([3, 1, 2], (3, 1, 2), np.array([3, 1, 2]), torch.tensor([3, 1, 2]), [torch.tensor(3), np.int64(1), 2]):
+        got = _token_ids(ids)
+        assert got.dtype == torch.int32 and got.tolist() == [3, 1, 2]
+    assert _token_ids([]).shape == (0,)
+    for bad in ([2**31], np.array([2**32 + 5]), ["3"], [np.float32(1.5)]):
+        with pytest.raises((RuntimeError, ValueError, TypeError)):
+            _token_ids(bad)

@@ -44,9 +44,3 @@ def native_int32(values) -> np.ndarray | None:
         if lib.b200_host_fill_row(values, out.ctypes.data, len(values)) == 0:
             return out
     return None
-
-
-def as_int32(values) -> np.ndarray:
-    """``np.asarray(values, dtype=np.int32)``."""
-    fast = native_int32(values)
-    return np.asarray(values, dtype=np.int32) if fast is None else fast

@@ -22,7 +22,7 @@ import torch
 from ..attention.context import clear_context, get_context, prepare_grouped, prepare_unified
 from ..attention.impls.sdpa import _KernelMetadata, _kernel_metadata
 from ..attention.impls.segments import SegmentMetadata
-from ..host_lists import as_int32, fill_rows
+from ..host_lists import fill_rows, native_int32
 from ..metal import get_ops
 from ..metal.constants import PARTITION_SIZE
 
@@ -79,6 +79,13 @@ class StepBuffers:
     def upload(self) -> int:
         self.dev.copy_(self.host, non_blocking=True)
         return self.words * 4
+
+
+def _token_ids(input_ids: Sequence[int]) -> torch.Tensor:
+    """int32 on the host, of whatever ``torch.tensor`` takes: integers, scalars of a device, NumPy's."""
+    ids = list(input_ids)
+    fast = native_int32(ids)
+    return torch.tensor(ids, dtype=torch.int32) if fast is None else torch.from_numpy(fast)
 
 
 class _PendingTokens:
@@ -158,7 +165,7 @@ class PagedModelRunner:
                 ctx.state_slots = list(state_slots)
             if rows is None:
                 rows = [c - 1 for c in ctx.cu_seqlens[1:]]
-            ids = torch.from_numpy(as_int32(list(input_ids))).pin_memory().to(self.device, non_blocking=True)
+            ids = _token_ids(input_ids).pin_memory().to(self.device, non_blocking=True)
             row_ids = torch.tensor(list(rows), dtype=torch.int64).pin_memory().to(self.device, non_blocking=True)
             self.last_logits = self.model(ids, ctx, self.kv_cache, logits_rows=row_ids)
             # bytes that crossed PCIe for this step: ids + logit rows + the kernel metadata sdpa uploads once
@@ -213,7 +220,7 @@ class PagedModelRunner:
             prepare_unified(reqs, [], self.block_size, merge_verify_windows=self.merge_verify_windows)
         ctx = get_context()
         try:
-            ids = torch.from_numpy(as_int32(list(input_ids))).pin_memory().to(self.device, non_blocking=True)
+            ids = _token_ids(input_ids).pin_memory().to(self.device, non_blocking=True)
             self.last_verify_logits = self.model(ids, ctx, self.kv_cache, logits_rows=None)
             toks = self._greedy(self.last_verify_logits).cpu().tolist()
             nseq = len(ctx.cu_seqlens) - 1
