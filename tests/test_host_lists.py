@@ -1,5 +1,7 @@
 """Rows of page numbers into int32 tables: the native conversion and the general one agree, and refuse the same."""
 
+import collections
+
 import numpy as np
 import pytest
 
@@ -111,3 +113,13 @@ def test_token_ids_as_torch_takes_them():
     for bad in ([2**31], np.array([2**32 + 5]), ["3"], [np.float32(1.5)]):
         with pytest.raises((RuntimeError, ValueError, TypeError)):
             _token_ids(bad)
+
+
+@pytest.mark.parametrize("kind", [list, tuple, np.array, collections.deque])
+@pytest.mark.parametrize("first,count", [(0, 1), (37, 40), (600, 40), (5, 0), (-3, 5)])
+def test_slots_of_any_sequence_of_pages(kind, first, count):
+    from vllm_metal_b200.attention.context import _slots
+
+    ids = list(range(100, 140))
+    want = [ids[p // 16] * 16 + p % 16 for p in range(first, first + count)]
+    assert _slots(kind(ids), first, count, 16) == want

@@ -71,8 +71,11 @@ def clear_context() -> None:
 def _slots(block_ids: Sequence[int], first: int, count: int, block_size: int) -> list[int]:
     """Flat cache slots of positions ``first .. first+count-1`` of one request."""
     pos = np.arange(first, first + count, dtype=np.int64)
-    low = max(0, first) // block_size  # the pages of these positions alone: a long request has many more
-    ids = np.asarray(block_ids[low:(first + count - 1) // block_size + 1], dtype=np.int64)
+    low = 0
+    if first >= 0 and isinstance(block_ids, (list, tuple, np.ndarray)):  # the pages of these positions alone: a request may have many more
+        low = first // block_size
+        block_ids = block_ids[low:(first + count - 1) // block_size + 1]
+    ids = np.asarray(block_ids, dtype=np.int64)
     return (ids[pos // block_size - low] * block_size + pos % block_size).tolist()
 
 
