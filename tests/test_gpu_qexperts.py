@@ -188,3 +188,23 @@ def test_routers_that_are_no_buffers_of_a_router():
     del blk.router
     blk.router = lambda z: z @ w.t()
     torch.testing.assert_close(blk(x), plain, rtol=2**-6, atol=2e-3)
+
+
+def test_reads_back_to_the_host():
+    """The block none, the experts with choices from elsewhere one."""
+    import warnings
+
+    blk = _block(128, 64, 7, 2, 4, 64, "silu", "topk_softmax", False)
+    x = torch.randn((9, 128), device="cuda").bfloat16()
+    idx = blk.route(x)[0]
+    for call, most in ((lambda: blk(x), 0), (lambda: blk.experts(x, idx), 1)):
+        call()
+        torch.cuda.synchronize()
+        with warnings.catch_warnings(record=True) as seen:
+            warnings.simplefilter("always")
+            torch.cuda.set_sync_debug_mode("warn")
+            try:
+                call()
+            finally:
+                torch.cuda.set_sync_debug_mode("default")
+        assert sum("called a synchronizing" in str(w.message) for w in seen) <= most

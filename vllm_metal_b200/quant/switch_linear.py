@@ -222,7 +222,7 @@ class SwitchGLU(nn.Module):
         t, k = indices.shape
         tile_rows = self.grouped_tile_rows(x, k) if x.dim() == 2 and x.shape[0] == t and k else 0
         if tile_rows:
-            lo, hi = (int(v) for v in torch.aminmax(indices))
+            lo, hi = torch.stack(torch.aminmax(indices)).tolist()  # the one host read-back of this form
             if lo < 0 or hi >= self.gate_proj.num_experts:
                 raise ValueError(f"expert indices must lie in [0, {self.gate_proj.num_experts}), got {lo} .. {hi}")
             return self.grouped(x, indices.to(torch.int32), tile_rows).reshape(t, k, -1)
