@@ -247,7 +247,9 @@ int b200_qlinear_experts(const void* x, const uint32_t* w, const void* scales, c
  *   b200_qexpert_product gated = 1: out[i, :] (fp16, same column order as x) = act(gate, up) of row i, both rounded to bf16;
  *                        activation 0 silu(g) u, 1 clipped SwiGLU (alpha 1.702, limit 7).  gated = 0: out[pairs[i], :] (bf16).
  *   b200_qexpert_sum     out [rows, cols] = sum_j weights[row, j] y[row * top + j, :], fp32 sums in the order of j
- *   b200_qexpert_failed  synchronises; 1 if a plan did not fit together or a bounded wait ran out (results invalid), else 0 */
+ *   b200_qexpert_status  1 if, since the last reset, a plan did not fit together or a bounded wait ran out in a product that has
+ *                        finished, in this process, else 0; does not wait.  What such a product did not compute is NaN.
+ *   b200_qexpert_failed  the same after waiting for the device; no reset */
 typedef struct b200_qexpert_product_args {
   const void* x;      /* fp16 [total, k], sorted by expert */
   const uint32_t* w;  /* [experts, n_out, k * bits / 32] */
@@ -271,6 +273,7 @@ int b200_qexpert_rows(const void* x, const int32_t* pairs, void* y, int total, i
                       void* stream);
 int b200_qexpert_product(const b200_qexpert_product_args* a, void* stream);
 int b200_qexpert_sum(const void* y, const float* weights, void* out, int rows, int top, int cols, void* stream);
+int b200_qexpert_status(int reset);
 int b200_qexpert_failed(void);
 /* All of it in one call: out [rows, width] = the block's result for x [rows, width] (bf16, x_stride elements apart).  The router is
  * bf16 [experts, width].  B200_ERR_UNSUPPORTED for sizes that the parts above do not take (nothing was enqueued). */

@@ -208,3 +208,78 @@ def test_reads_back_to_the_host():
             finally:
                 torch.cuda.set_sync_debug_mode("default")
         assert sum("called a synchronizing" in str(w.message) for w in seen) <= most
+
+
+def _product_operands(tokens=40, hidden=128, inter=192, experts=7, top=2, bits=4):
+    from vllm_metal_b200.metal import get_ops
+
+    ops, blk = get_ops(), _block(hidden, inter, experts, top, bits, 64, "silu", "topk_softmax", False)
+    x = torch.randn((tokens, hidden), device="cuda").bfloat16()
+    tile_rows = blk.experts.grouped_tile_rows(x, top)
+    plan = ops.expert_plan(blk.route(x)[0].int().contiguous(), experts, tile_rows)
+    return ops, blk.experts, plan, ops.qexpert_rows(x, plan[0], top, bits)
+
+
+def _spoilt(plan, what):
+    """The plan with running counts that do not fit together."""
+    first, tiles = plan[1].clone(), plan[2].clone()
+    if what == "a tile too many":
+        tiles[1:] += 1
+    elif what == "counts that fall":
+        first[2] = first[3] + 5
+    elif what == "more tiles than there can be":
+        tiles[-1] = 10**6
+    elif what == "a negative row":
+        first[1] = -4
+    return plan[0], first, tiles, plan[3]
+
+
+@pytest.mark.parametrize("what", ["a tile too many", "counts that fall", "more tiles than there can be", "a negative row"])
+def test_a_plan_that_does_not_fit_together(what):
+    """Nothing is touched that the plan leads to, the results are NaN, the status says so until it is reset, and the next call is
+    sound."""
+    ops, glu, plan, xs = _product_operands()
+    assert not ops.qexpert_failed()
+    want = ops.qexpert_product(xs, glu.gate_proj, plan, up=glu.up_proj)
+    down = ops.qexpert_product(want, glu.down_proj, plan)
+    assert torch.isfinite(want).all() and torch.isfinite(down).all()
+    bad = _spoilt(plan, what)
+    try:
+        h = ops.qexpert_product(xs, glu.gate_proj, bad, up=glu.up_proj)
+        torch.cuda.current_stream().synchronize()
+        assert ops.qexpert_status() and torch.isnan(h).all()
+        assert ops.qexpert_status(reset=True) and not ops.qexpert_failed()
+        assert torch.isnan(ops.qexpert_product(want, glu.down_proj, bad)).all()
+        assert ops.qexpert_failed()
+        assert torch.isnan(ops.qexpert_product(h, glu.down_proj, plan)).all()  # what follows shows it
+    finally:
+        torch.cuda.synchronize()
+        ops.qexpert_status(reset=True)
+    assert torch.equal(ops.qexpert_product(xs, glu.gate_proj, plan, up=glu.up_proj), want)
+    assert not ops.qexpert_failed()
+
+
+def test_a_step_after_a_failed_product_raises():
+    import dataclasses
+
+    from vllm_metal_b200.attention.caches.kv_cache import B200PagedKVCache
+    from vllm_metal_b200.lm.decoder import PRESETS, Model
+    from vllm_metal_b200.v1.model_runner import PagedModelRunner
+
+    args = dataclasses.replace(PRESETS["tiny"], num_experts=4, experts_per_tok=2)
+    cache = B200PagedKVCache(args.num_layers, args.n_kv_heads, args.head_dim, 4, 16, torch.bfloat16, "cuda",
+                             sliding_window_per_layer=args.sliding_window_per_layer())
+    runner = PagedModelRunner(Model(args, torch.bfloat16, "cuda", seed=0), cache, max_batch=1, max_model_len=32)
+    ids, table = list(range(1, 9)), [1]
+    want = runner.execute(ids, [], [(table, 8, 0)])
+    ops, glu, plan, xs = _product_operands()
+    try:
+        ops.qexpert_product(xs, glu.gate_proj, _spoilt(plan, "a tile too many"), up=glu.up_proj)
+        for step in (lambda: runner.execute(ids, [], [(table, 8, 0)]), lambda: runner.verify(ids, [(table, 0, 8)]),
+                     lambda: runner.decode_step([1], [table], [8]), lambda: runner.submit_decode([1], [table], [8]).tokens()):
+            with pytest.raises(RuntimeError, match="grouped expert product"):
+                step()
+    finally:
+        torch.cuda.synchronize()
+        ops.qexpert_status(reset=True)
+    assert runner.execute(ids, [], [(table, 8, 0)]) == want

@@ -24,7 +24,9 @@
 #include "qdequant.cuh"
 #include "tcgen05.cuh"
 
+#include <atomic>
 #include <cmath>
+#include <mutex>
 
 namespace b200 {
 namespace qx {
@@ -39,8 +41,6 @@ constexpr int kMaxExperts = 1024;
 constexpr int kBarBytes = 704;
 constexpr int kDqg = 1, kEpg = 2;   // sets of unpacking warps (two gained nothing) and of epilogue warps (one: 183 us instead of 169)
 
-__device__ int g_failed = 0;  // a wait ran out or the plan was not sound: results of the launch are invalid
-
 struct Params {
   const int32_t *pairs, *first, *tiles;
   const uint16_t* scales[2];  // gated: gate, up
@@ -50,7 +50,29 @@ struct Params {
   int64_t out_stride;
   int total, experts, n_out, groups, num_kb, max_tiles;
   int cap, box, ps, nx, na, nbuf, act;
+  int* status;  // on the host; set to 1 if a wait ran out or the plan did not fit together
 };
+
+// That word, one for the process: a launch that fails writes it, the host looks after it has waited for the stream anyway.
+static int* status_word(bool make) {
+  static std::atomic<int*> word{nullptr};
+  static std::mutex lock;
+  int* w = word.load(std::memory_order_acquire);
+  if (w || !make) return w;
+  std::lock_guard<std::mutex> hold(lock);
+  w = word.load(std::memory_order_acquire);
+  if (w) return w;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // an allocation is no part of a capture that may be under way
+  const bool swapped = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+  void* p = nullptr;
+  const cudaError_t e = cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped);
+  if (swapped) cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) return nullptr;
+  w = static_cast<int*>(p);
+  *w = 0;
+  word.store(w, std::memory_order_release);
+  return w;
+}
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
@@ -166,7 +188,8 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   tc_fence_after();
   const uint32_t tmem = *tmem_gen;
   const int ft = (p.n_out + FEATURES - 1) / FEATURES;
-  const int items = *sfail ? 0 : tiles[p.experts] * ft;
+  const bool sound = *sfail == 0;
+  const int items = sound ? tiles[p.experts] * ft : 0;
   __syncthreads();
   bool ok = true;
 
@@ -454,7 +477,28 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   }
   tc_fence_before();
   __syncthreads();
-  if (*sfail && threadIdx.x == 0) atomicExch(&g_failed, 1);
+  if (*sfail) {
+    // What should have been written here is NaN (0x7fff in both types), never what the memory held: everything for a plan that
+    // does not fit together, else this CTA's items.
+    const uint32_t nan2 = 0x7fff7fffu;
+    auto fill = [&](int64_t row, int col) { *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(p.out) + row * p.out_stride + col) = nan2; };
+    if (!sound) {
+      const int half = p.n_out / 2;
+      for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)p.total * half; i += (int64_t)gridDim.x * blockDim.x)
+        fill(i / half, (int)(i % half) * 2);
+    }
+    for (int i = blockIdx.x; i < items; i += gridDim.x) {
+      const Item w = item_at<FEATURES>(p, tiles, first, ft, i);
+      for (int j = threadIdx.x; j < w.nrows * (FEATURES / 2); j += blockDim.x) {
+        const int r = w.row0 + j / (FEATURES / 2), c = w.n0 + j % (FEATURES / 2) * 2;
+        if (c < p.n_out) fill(GATED ? r : (int64_t)min((uint32_t)p.pairs[r], (uint32_t)p.total - 1), c);
+      }
+    }
+    if (threadIdx.x == 0) {
+      *reinterpret_cast<volatile int*>(p.status) = 1;
+      __threadfence_system();
+    }
+  }
   if (warp == W_MMA) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
@@ -702,6 +746,8 @@ static int launch_steps(const b200_qexpert_product_args& a, const Rings& ring, c
   p.na = (512 - 2 * ring.cap) / (32 * SK) < kMaxA ? (512 - 2 * ring.cap) / (32 * SK) : kMaxA;
   p.nbuf = ring.nbuf;
   p.act = a.activation;
+  p.status = status_word(true);
+  if (!p.status) return set_error(B200_ERR_CUDA, "qexpert_product: no pinned memory for the status word");
   constexpr int FEATURES = GATED ? 64 : 128;
   const int64_t items = (int64_t)p.max_tiles * ((a.n_out + FEATURES - 1) / FEATURES);
   const int sms = sm_count() > 0 ? sm_count() : 148;
@@ -762,11 +808,15 @@ int b200_qexpert_product(const b200_qexpert_product_args* a, void* stream) {
   return a->gated ? qx::dispatch<true>(*a, r, (cudaStream_t)stream) : qx::dispatch<false>(*a, r, (cudaStream_t)stream);
 }
 
-int b200_qexpert_failed(void) {
-  int v = 0;
-  if (cudaMemcpyFromSymbol(&v, qx::g_failed, sizeof(v)) != cudaSuccess) return 1;
+int b200_qexpert_status(int reset) {
+  volatile int* w = qx::status_word(false);
+  if (!w) return 0;
+  const int v = *w;
+  if (reset) *w = 0;
   return v;
 }
+
+int b200_qexpert_failed(void) { return cudaDeviceSynchronize() != cudaSuccess ? 1 : b200_qexpert_status(0); }
 
 int b200_qexpert_rows(const void* x, const int32_t* pairs, void* y, int total, int top, int cols, int64_t x_stride, int permute, void* stream) {
   B200_CHECK_ARG(x && pairs && y && top >= 1 && cols >= 8 && cols % 8 == 0 && x_stride % 8 == 0 && qx::aligned(x) && qx::aligned(y),

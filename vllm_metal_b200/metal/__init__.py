@@ -137,6 +137,7 @@ EXPORTED_SYMBOLS = (
     "b200_qexpert_rows",
     "b200_qexpert_product",
     "b200_qexpert_sum",
+    "b200_qexpert_status",
     "b200_qexpert_failed",
     "b200_qexpert_block",
     "b200_qexpert_block_workspace_bytes",
@@ -723,8 +724,13 @@ class _Ops(HybridOps):
         self.launches += 6
         return out
 
+    def qexpert_status(self, reset: bool = False) -> bool:
+        """Whether a grouped product that has finished has failed (its plan did not fit together, a wait ran out) in this process
+        since the last ``reset``; its results are NaN.  Reads a word of host memory: look after a wait for the stream."""
+        return self._lib.b200_qexpert_status(int(reset)) != 0
+
     def qexpert_failed(self) -> bool:
-        """Whether a wait inside the grouped product kernel ever ran out (synchronises)."""
+        """The same after waiting for the device."""
         return self._lib.b200_qexpert_failed() != 0
 
     def qlinear_prepack(self, w, bits: int = 4, inverse: bool = False, out=None):

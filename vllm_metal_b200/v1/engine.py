@@ -222,6 +222,8 @@ class Engine:
             return []
         done: list[Request] = []
         tokens = self.runner._greedy(self._run(work, None)).tolist()
+        if getattr(self.runner, "has_moe", False):
+            self.runner._check_experts()
         for (req, _), token in zip(work, tokens, strict=True):
             if req.num_computed < len(req.tokens):
                 continue  # a portion that does not reach the end of the prompt samples nothing

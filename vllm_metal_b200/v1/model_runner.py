@@ -91,13 +91,15 @@ def _token_ids(input_ids: Sequence[int]) -> torch.Tensor:
 class _PendingTokens:
     """Tokens of a submitted decode step; ``tokens()`` waits for the read-back."""
 
-    def __init__(self, event, host: torch.Tensor, n: int) -> None:
-        self._event, self._host, self._n = event, host, n
+    def __init__(self, event, host: torch.Tensor, n: int, check=None) -> None:
+        self._event, self._host, self._n, self._check = event, host, n, check
         self._tokens: list[int] | None = None
 
     def tokens(self) -> list[int]:
         if self._tokens is None:
             self._event.synchronize()
+            if self._check is not None:
+                self._check()
             self._tokens = self._host[: self._n].tolist()
         return self._tokens
 
@@ -115,6 +117,7 @@ class PagedModelRunner:
         # blocks of sizes that the grouped expert kernels do not take read row counts back to the host: not capturable
         has_moe = any(hasattr(getattr(layer, "mlp", None), "block") for layer in getattr(model, "layers", []))
         self.use_cuda_graph = use_cuda_graph and not has_moe
+        self.has_moe = has_moe
         # recurrent layers: every request owns a state slot, named by the caller step for step
         self.stateful = bool(getattr(model, "stateful", False))
         self.last_logits: torch.Tensor | None = None  # of the last step: one row per segment / per requested row
@@ -131,6 +134,12 @@ class PagedModelRunner:
         greedy = getattr(self.model, "greedy", None)  # vocab-parallel heads exchange (max, id) between the ranks
         return greedy(logits, out=out) if greedy is not None else get_ops().argmax(logits, out=out)
 
+    def _check_experts(self) -> None:
+        """After a step's read-back: a grouped expert product that failed has left NaN, from which tokens are not to be taken."""
+        if self.has_moe and get_ops().qexpert_status():
+            raise RuntimeError("a grouped expert product has failed: results since are not valid "
+                               "(get_ops().qexpert_status(reset=True) starts anew)")
+
     # -- generic (eager) path: any mix of prefill chunks and decode rows -----------
     def execute(self, input_ids: Sequence[int], decode_requests, prefill_requests,
                 state_slots: Sequence[int] | None = None) -> list[int]:
@@ -142,6 +151,7 @@ class PagedModelRunner:
         """
         logits = self.forward_rows(input_ids, decode_requests, prefill_requests, None, state_slots)
         out = self._greedy(logits).cpu().tolist()
+        self._check_experts()
         self.d2h_bytes += len(out) * 4
         return out
 
@@ -223,6 +233,7 @@ class PagedModelRunner:
             ids = _token_ids(input_ids).pin_memory().to(self.device, non_blocking=True)
             self.last_verify_logits = self.model(ids, ctx, self.kv_cache, logits_rows=None)
             toks = self._greedy(self.last_verify_logits).cpu().tolist()
+            self._check_experts()
             nseq = len(ctx.cu_seqlens) - 1
             maxb = max((len(t) for t in (ctx.block_tables or [])), default=0)
             self.h2d_bytes += ids.numel() * 4 + len(ctx.slot_mapping) * 12 + (2 * nseq + 1) * 4 + nseq * maxb * 4
@@ -300,6 +311,7 @@ class PagedModelRunner:
         self.d2h_bytes += n * 4
         if sync:
             torch.cuda.current_stream().synchronize()
+            self._check_experts()
             return self.buf.out_host[:n].tolist()
         return None
 
@@ -339,7 +351,7 @@ class PagedModelRunner:
         self.d2h_bytes += n * 4
         ev = torch.cuda.Event()
         ev.record()
-        return _PendingTokens(ev, host, n)
+        return _PendingTokens(ev, host, n, self._check_experts)
 
     def run_decode(self, batch: int, max_seq_len: int, *, advance: bool = False) -> None:
         """Forward + argmax over the persistent buffers (graph replay when enabled).
