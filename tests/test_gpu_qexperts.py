@@ -231,10 +231,17 @@ def _spoilt(plan, what):
         tiles[-1] = 10**6
     elif what == "a negative row":
         first[1] = -4
+    elif what == "tiles that start late":
+        tiles += 1
+    elif what == "rows that start late":
+        first[0] = 1
+    elif what == "rows that end early":
+        first[-1] -= 1
     return plan[0], first, tiles, plan[3]
 
 
-@pytest.mark.parametrize("what", ["a tile too many", "counts that fall", "more tiles than there can be", "a negative row"])
+@pytest.mark.parametrize("what", ["a tile too many", "counts that fall", "more tiles than there can be", "a negative row",
+                                  "tiles that start late", "rows that start late", "rows that end early"])
 def test_a_plan_that_does_not_fit_together(what):
     """Nothing is touched that the plan leads to, the results are NaN, the status says so until it is reset, and the next call is
     sound."""

@@ -173,14 +173,15 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   }
   __syncthreads();
   pdl_wait();
-  // The plan is checked on the way in: running counts that fit together, so that whatever they hold, every row below is a
-  // row of the operands.
+  // The plan is checked on the way in: running counts from nought to all rows that fit together, so that whatever they hold, every
+  // row below is a row of the operands and every row of the result is written.
   for (int i = threadIdx.x; i <= p.experts; i += blockDim.x) {
     const int t = p.tiles[i], f = p.first[i];
     tiles[i] = t;
     first[i] = f;
     const int tn = i < p.experts ? p.tiles[i + 1] : t, fn = i < p.experts ? p.first[i + 1] : p.total;
-    if (t < 0 || f < 0 || t > p.max_tiles || f > p.total || (i < p.experts && (fn < f || tn - t != (fn - f + p.cap - 1) / p.cap)))
+    if (t < 0 || f < 0 || t > p.max_tiles || f > p.total || (i == 0 && (t != 0 || f != 0)) || (i == p.experts && f != p.total) ||
+        (i < p.experts && (fn < f || tn - t != (fn - f + p.cap - 1) / p.cap)))
       *sfail = 1;
   }
   tc_fence_before();
