@@ -365,3 +365,25 @@ def test_products_refuse_what_they_cannot_do(ops):
         ops.expert_route(torch.zeros((2, 4), device="cuda"), None, 4, 5, 1.0)
     with pytest.raises(RuntimeError, match="CUDA"):
         ops.expert_route(torch.zeros((2, 4)), None, 4, 2, 1.0)
+
+
+@pytest.mark.parametrize("what", ["tiles[:] += 1", "first[0] = 1", "first[-1] -= 1"])
+def test_plans_that_do_not_start_at_nought_are_seen(what):
+    """By the status, in a process of its own since it stays; the plan leads nowhere."""
+    import subprocess
+    import sys
+
+    code = f"""
+import torch
+from vllm_metal_b200.metal import get_ops
+ops = get_ops()
+x, w = (torch.randn(s, device="cuda").bfloat16() for s in ((64, 64), (5, 128, 64)))
+pairs, first, tiles, rows = ops.expert_plan(torch.randint(0, 5, (64, 2), device="cuda").int(), 5, 64)
+ops.expert_product(x, w, (pairs, first, tiles, rows), 2, 64, gated=True, kernel=2)
+assert not ops.expert_product_failed()
+{what}
+ops.expert_product(x, w, (pairs, first, tiles, rows), 2, 64, gated=True, kernel=2)
+torch.cuda.synchronize()
+assert ops.expert_product_failed()
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=120)

@@ -147,15 +147,16 @@ expert_product_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   pdl_wait();
-  // The plan is checked on the way in: running counts that fit together, so that whatever they hold, every row below is
-  // a row of the operands.
+  // The plan is checked on the way in: running counts from nought to all pairs that fit together, so that whatever they hold, every
+  // row below is a row of the operands.
   const int pairs_total = p.rows * p.top;
   for (int i = threadIdx.x; i <= p.experts; i += blockDim.x) {
     const int t = p.tiles[i], f = p.first[i];
     tiles[i] = t;
     first[i] = f;
     const int tn = i < p.experts ? p.tiles[i + 1] : t, fn = i < p.experts ? p.first[i + 1] : pairs_total;
-    if (t < 0 || f < 0 || t > p.max_tiles || f > pairs_total || (i < p.experts && (fn < f || tn - t != (fn - f + TOKENS - 1) / TOKENS)))
+    if (t < 0 || f < 0 || t > p.max_tiles || f > pairs_total || (i == 0 && (t != 0 || f != 0)) || (i == p.experts && f != pairs_total) ||
+        (i < p.experts && (fn < f || tn - t != (fn - f + TOKENS - 1) / TOKENS)))
       *sfail = 1;
   }
   tc_fence_before();
