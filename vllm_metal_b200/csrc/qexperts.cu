@@ -5,9 +5,9 @@
 // features on the way out) and an expert's rows the N side (16 .. 192 of them, in steps of 16: its rows are split evenly over
 // as few tiles as hold them), so packed weights cross HBM once and are unpacked once for up to 192 rows.
 //
-//   warps 0 .. 8 DQG - 1   unpack: half a weight row of 64 columns a thread; int4 / int8 -> s * q + b (one rounding to fp16)
+//   8 warps                unpack: half a weight row of 64 columns a thread; int4 / int8 -> s * q + b (one rounding to fp16)
 //                          -> the A ring in tensor memory
-//   4 EPG warps            epilogue: bias, activation, stores; two accumulators, so the next item's products overlap it
+//   8 warps                epilogue: bias, activation, stores; two accumulators, so the next item's products overlap it
 //   1 warp                 packed words (ring) and the whole rows' scales and biases of an item (one bulk copy each: rows are
 //                          contiguous, however odd K / group is)
 //   1 warp                 the rows of x, by TMA from the grouped fp16 copy
@@ -39,7 +39,9 @@ constexpr int kMaxTile = 192;       // rows of x a tile holds: two accumulators 
 constexpr int kSmemMax = 232448;
 constexpr int kMaxExperts = 1024;
 constexpr int kBarBytes = 704;
-constexpr int kDqg = 1, kEpg = 2;   // sets of unpacking warps (two gained nothing) and of epilogue warps (one: 183 us instead of 169)
+constexpr int kUnpackWarps = 8;     // a second set gained nothing
+constexpr int kEpiSets = 2;         // sets of four epilogue warps; one: 183 us instead of 169
+constexpr int kThreads = kUnpackWarps * 32 + kEpiSets * 128 + 96;
 
 struct Params {
   const int32_t *pairs, *first, *tiles;
@@ -121,20 +123,20 @@ __device__ __forceinline__ float activate(int act, float g, float u) {
 }
 
 // SK: 64-column blocks of a step of the A ring and of x.
-template <int BITS, int G, bool GATED, int SK, int DQG, int EPG>
-__global__ void __launch_bounds__(DQG * 256 + EPG * 128 + 96, 1)
+template <int BITS, int G, bool GATED, int SK>
+__global__ void __launch_bounds__(kThreads, 1)
 expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap u_map,
                     const __grid_constant__ CUtensorMap x_map, const Params p) {
   constexpr int FEATURES = GATED ? 64 : 128, A_COLS = 32 * SK;
   constexpr int KB_PER_P = 1024 / BITS / 64;     // 64-column blocks of a packed stage
   constexpr int U = SK < 2 ? SK : 2;             // that a thread unpacks at a time
   constexpr int CH_T = BITS / 4;                 // 16-byte packed chunks a thread unpacks per block
-  constexpr int W_EPI = 8 * DQG, W_W = W_EPI + 4 * EPG, W_X = W_W + 1, W_MMA = W_W + 2;
+  constexpr int W_EPI = kUnpackWarps, W_W = W_EPI + 4 * kEpiSets, W_X = W_W + 1, W_MMA = W_W + 2;
   extern __shared__ __align__(1024) uint8_t raw[];
   const uint32_t base = (smem_u32(raw) + 1023u) & ~1023u;
   const uint32_t xb = p.cap * 128 * SK, row_bytes = p.groups * 2, half_sb = 128 * row_bytes, sb_bytes = 2 * half_sb;
   const uint32_t sm_x = base + p.ps * kPacked, sm_sb = sm_x + p.nx * xb, sm_ex = sm_sb + p.nbuf * sb_bytes;
-  const uint32_t sm_bar = sm_ex + (GATED ? EPG * 8192 : 0);
+  const uint32_t sm_bar = sm_ex + (GATED ? kEpiSets * 8192 : 0);
   const uint32_t bar_full_p = sm_bar, bar_empty_p = bar_full_p + 64, bar_full = bar_empty_p + 64, bar_empty = bar_full + 8 * kMaxA;
   const uint32_t bar_acc = bar_empty + 8 * kMaxA, bar_free = bar_acc + 16, bar_full_sb = bar_free + 16, bar_empty_sb = bar_full_sb + 16;
   const uint32_t bar_full_x = bar_empty_sb + 16, bar_empty_x = bar_full_x + 8 * kMaxX, tmem_ptr = bar_empty_x + 8 * kMaxX;
@@ -148,7 +150,7 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   if (threadIdx.x == 0) {
     for (int i = 0; i < p.ps; ++i) {
       mbar_init(bar_full_p + 8 * i, 1);
-      mbar_init(bar_empty_p + 8 * i, 8 * DQG);
+      mbar_init(bar_empty_p + 8 * i, kUnpackWarps);
     }
     for (int i = 0; i < p.na; ++i) {
       mbar_init(bar_full + 8 * i, 8);
@@ -160,9 +162,9 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar_acc + 8 * i, 1);
-      mbar_init(bar_free + 8 * i, 4 * EPG);
+      mbar_init(bar_free + 8 * i, 4 * kEpiSets);
       mbar_init(bar_full_sb + 8 * i, 1);
-      mbar_init(bar_empty_sb + 8 * i, 8 * DQG);
+      mbar_init(bar_empty_sb + 8 * i, kUnpackWarps);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *sfail = 0;
@@ -311,10 +313,10 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     }
     if (!ok && lane == 0) *sfail = 1;
   } else if (warp < W_EPI) {
-    // ===== unpack; with two sets of warps each takes every second step =====
-    const int r = threadIdx.x & 127, hsel = (threadIdx.x >> 7) & 1, set = warp >> 3;
+    // ===== unpack =====
+    const int r = threadIdx.x & 127, hsel = (threadIdx.x >> 7) & 1;
     const uint32_t xr = r & 7, tm_a = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 2 * p.cap + hsel * 16;
-    int pst = 0, it = 0, slot = 0, turn = 0;
+    int pst = 0, it = 0, slot = 0;
     uint32_t pph = 0, sph = 1;
     for (int i = blockIdx.x; ok && i < items; i += gridDim.x, ++it) {
       const int buf = p.nbuf == 2 ? it & 1 : 0, use = p.nbuf == 2 ? it >> 1 : it;
@@ -329,15 +331,6 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           if (kb >= p.num_kb) continue;
           const int part = (kb / U) % (SK / U);  // of the step
           const bool last = part == SK / U - 1 || kb + U >= p.num_kb;
-          auto next = [&] {
-            if (!last) return;
-            turn ^= 1;
-            if (++slot == p.na) slot = 0, sph ^= 1;
-          };
-          if (DQG == 2 && turn != set) {
-            next();
-            continue;
-          }
           uint4 pk[U][CH_T];
           uint16_t sr[U], br[U];
 #pragma unroll
@@ -381,8 +374,8 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_full + 8 * slot);
+            if (++slot == p.na) slot = 0, sph ^= 1;
           }
-          next();
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_empty_p + 8 * pst);
@@ -394,7 +387,7 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     if (!ok && lane == 0) *sfail = 1;
   } else {
     // ===== epilogue: thread = weight row of the tile; the sets of four warps take columns in turn =====
-    const int q = warp & 3, r = q * 32 + lane, set = EPG == 2 ? (warp - W_EPI) >> 2 : 0;
+    const int q = warp & 3, r = q * 32 + lane, set = (warp - W_EPI) >> 2;
     const uint32_t tm = tmem + ((uint32_t)(q * 32) << 16);
     int it = 0, flip = 0;
     for (int i = blockIdx.x; i < items; i += gridDim.x, ++it) {
@@ -414,7 +407,7 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       const uint32_t d = tm + (it & 1) * p.cap;
       if constexpr (GATED) {
         __half* out = reinterpret_cast<__half*>(p.out);
-        for (int c0 = set * 32; c0 < w.nrows; c0 += 32 * EPG) {
+        for (int c0 = set * 32; c0 < w.nrows; c0 += 32 * kEpiSets) {
           uint32_t mine[16], other[16] = {};
           // gate lanes finish the first 16 columns, up lanes the second: each hands its other 16 over
           const bool second = c0 + 16 < w.nrows;  // the last 32 columns may hold one sixteen only
@@ -455,7 +448,7 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       } else {
         __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + (feature & ~1);
         const bool odd = lane & 1, live = feature < p.n_out;
-        for (int c0 = set * 16; c0 < w.nrows; c0 += 16 * EPG) {
+        for (int c0 = set * 16; c0 < w.nrows; c0 += 16 * kEpiSets) {
           uint32_t u[16];
           tmem_ld<16>(d + c0, u);
           const int place = (int)min((uint32_t)p.pairs[w.row0 + min(c0 + (lane & 15), w.nrows - 1)], (uint32_t)p.total - 1);
@@ -675,7 +668,7 @@ constexpr int kNumCaps = 7;
 static bool rings_of(Rings& o, int cap, int experts, int k, int group, bool gated) {
   const int sb = 2 * 128 * (k / group) * 2, sk = cap <= 64 ? 4 : 1, xb = cap * 128 * sk;
   for (int nbuf = 2; nbuf >= 1; --nbuf) {
-    const int room = kSmemMax - (1024 + nbuf * sb + (gated ? kEpg * 8192 : 0) + kBarBytes + 8 * (experts + 1));
+    const int room = kSmemMax - (1024 + nbuf * sb + (gated ? kEpiSets * 8192 : 0) + kBarBytes + 8 * (experts + 1));
     int ps = 3, nx = sk == 4 ? 2 : 4;
     if (room < ps * kPacked + nx * xb) continue;
     auto left = [&] { return room - ps * kPacked - nx * xb; };
@@ -703,7 +696,7 @@ static int choose_cap(int rows, int top, int experts, int k, int group, bool gat
 
 template <int BITS, int G, bool GATED, int SK>
 static int launch_steps(const b200_qexpert_product_args& a, const Rings& ring, cudaStream_t st) {
-  auto kern = expert_qgemm_kernel<BITS, G, GATED, SK, kDqg, kEpg>;
+  auto kern = expert_qgemm_kernel<BITS, G, GATED, SK>;
   static int configured[16] = {0};
   int dev = 0;
   B200_CUDA_OK(cudaGetDevice(&dev));
@@ -752,7 +745,7 @@ static int launch_steps(const b200_qexpert_product_args& a, const Rings& ring, c
   constexpr int FEATURES = GATED ? 64 : 128;
   const int64_t items = (int64_t)p.max_tiles * ((a.n_out + FEATURES - 1) / FEATURES);
   const int sms = sm_count() > 0 ? sm_count() : 148;
-  B200_CUDA_OK(launch_pdl(kern, dim3(items < sms ? (int)items : sms), dim3(kDqg * 256 + kEpg * 128 + 96), ring.smem, st, w, u, x, p));
+  B200_CUDA_OK(launch_pdl(kern, dim3(items < sms ? (int)items : sms), dim3(kThreads), ring.smem, st, w, u, x, p));
   return check_launch("expert_qgemm_kernel");
 }
 
