@@ -290,3 +290,69 @@ def test_a_step_after_a_failed_product_raises():
         torch.cuda.synchronize()
         ops.qexpert_status(reset=True)
     assert runner.execute(ids, [], [(table, 8, 0)]) == want
+
+
+@pytest.mark.parametrize("experts,top", [(32, 4), (33, 1), (64, 32), (65, 8), (128, 32), (129, 8)])
+@pytest.mark.parametrize("routing", ["topk_softmax", "softmax_topk"])
+def test_choice_over_more_experts(experts, top, routing):
+    """Rows and router of few bits, whose products and sums are exact in any order: the choices, of which many tie, are those of the
+    sort; 129 experts are more than the kernel takes."""
+    from vllm_metal_b200.metal import get_ops
+    from vllm_metal_b200.quant.switch_linear import MoEBlock, Router
+
+    g = torch.Generator(device="cuda").manual_seed(experts)
+    router = Router(96, experts, True, torch.bfloat16, "cuda")
+    router.weight.copy_(torch.randint(-2, 3, router.weight.shape, device="cuda", generator=g) / 4)
+    router.bias.copy_(torch.randint(-2, 3, router.bias.shape, device="cuda", generator=g) / 4)
+    x = torch.randint(-1, 2, (37, 96), device="cuda", generator=g).bfloat16()
+    before = get_ops().launches
+    idx, scores = MoEBlock(router, None, top, routing).route(x)
+    assert get_ops().launches - before == (experts <= 128)
+    logits = (x.double() @ router.weight.double().T + router.bias.double()).bfloat16().double()
+    vals, want = torch.sort(logits, dim=-1, descending=True, stable=True)
+    assert torch.equal(idx, want[:, :top])
+    part = torch.softmax(vals if routing == "softmax_topk" else vals[:, :top], -1)[:, :top]
+    # a few roundings of 32 bits, and an exponential of one or two of its last bits
+    torch.testing.assert_close(scores.double(), part / part.sum(-1, keepdim=True), rtol=16 * 2**-24, atol=0)
+
+
+@pytest.mark.parametrize("experts", [40, 100, 129])
+def test_blocks_of_more_experts(experts):
+    blk = _block(128, 64, experts, 3, 4, 64, "silu", "softmax_topk", True)
+    x = torch.randn((50, 128), device="cuda", generator=torch.Generator(device="cuda").manual_seed(0)).bfloat16()
+    # the operands round alike on both ways: what is left is the activation's last bit in 16, and the result's
+    torch.testing.assert_close(blk(x).float(), _by_parts(blk, x, *blk.route(x)), rtol=2**-7, atol=2**-7)
+
+
+@pytest.mark.parametrize("act", ["silu", "gpt_oss"])
+def test_operands_beyond_fp16_and_infinite_projections(act):
+    """Rows saturate at fp16's largest as the other path's; infinite gates and halves as the activations in fp32 have them."""
+    blk = _block(128, 64, 7, 2, 4, 64, act, "topk_softmax", True)
+    x = torch.randn((9, 128), device="cuda", generator=torch.Generator(device="cuda").manual_seed(0)).bfloat16()
+    x[2, :5], x[3, 7] = 1e5, -3e38
+    idx, scores = torch.arange(18, device="cuda").view(9, 2) % 7, torch.full((9, 2), 0.5, device="cuda")
+    inf = float("inf")
+    for e, (g, u) in enumerate([(inf, 0), (-inf, 0), (0, inf), (0, -inf), (inf, inf), (inf, -inf)]):
+        blk.experts.gate_proj.bias[e, e], blk.experts.up_proj.bias[e, e] = g, u
+    blk.route = lambda z: (idx, scores)  # the choices are given
+    got = (blk.experts(x, idx).float() * scores[..., None]).sum(1)
+    want = _by_parts(blk, x, idx, scores)
+    for r in range(9):  # NaN (an infinite gate's, times nought) becomes a finite operand of the way out on both ways
+        assert torch.isfinite(want[r]).all() and (got[r] - want[r]).norm() <= 2**-6 * want[r].norm()
+
+
+def test_rows_of_another_stream_and_passes_that_repeat():
+    blk = _block(320, 192, 7, 2, 4, 64, "gpt_oss", "topk_softmax", True)
+    x = torch.randn((200, 320), device="cuda").bfloat16()
+    want = blk(x)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        rows = torch.zeros((4096, 4096), device="cuda")
+        for _ in range(8):
+            rows = rows @ rows  # the rows are late
+        late = x + rows[0, 0].bfloat16()
+        got = [blk(late) for _ in range(3)]
+    other = blk(x)  # meanwhile
+    torch.cuda.synchronize()
+    assert torch.equal(other, want) and all(torch.equal(y, want) for y in got)
