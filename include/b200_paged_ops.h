@@ -237,7 +237,7 @@ int b200_qlinear_experts(const void* x, const uint32_t* w, const void* scales, c
 
 /* The same for all experts at once, without a host read-back (csrc/qexperts.cu): bf16 activations, scales, biases and bias; k and
  * n_out whole multiples of 64; operands 16-byte aligned and contiguous.
- *   b200_qexpert_route   logits = x . w^T (+ bias) in fp32, rounded to bf16; the `top` largest, best first, ties to the lower
+ *   b200_qexpert_route   logits = x . w^T (+ bias) in 32-bit sums (tensor cores), rounded to bf16; the `top` largest, best first, ties to the lower
  *                        number (NaN before all), to chosen [rows, top]; scores: softmax over the chosen ones, or with over_all = 1
  *                        over all experts before the choice, norm = 1: divided by their sum.  At most 128 experts, top <= 32.
  *   b200_expert_plan     (b200_hybrid_ops.h) with tile_rows = b200_qexpert_tile_rows(...) -- the smaller one, if several
@@ -245,7 +245,7 @@ int b200_qlinear_experts(const void* x, const uint32_t* w, const void* scales, c
  *   b200_qexpert_rows    y [total, cols] fp16 (saturated) = x[pairs[i] / top]; `permute` (4-bit weights): every eight columns in the
  *                        order 0 4 1 5 2 6 3 7, as the products expect theirs
  *   b200_qexpert_product gated = 1: out[i, :] (fp16, same column order as x) = act(gate, up) of row i, both rounded to bf16;
- *                        activation 0 silu(g) u, 1 clipped SwiGLU (alpha 1.702, limit 7).  gated = 0: out[pairs[i], :] (bf16).
+ *                        activation 0 silu(g) u, 1 clipped SwiGLU (alpha 1.702, limit 7), with fast exponentials.  gated = 0: out[pairs[i], :] (bf16).
  *   b200_qexpert_sum     out [rows, cols] = sum_j weights[row, j] y[row * top + j, :], fp32 sums in the order of j
  *   b200_qexpert_status  1 if, since the last reset, a plan did not fit together or a bounded wait ran out in a product that has
  *                        finished, in this process, else 0; does not wait.  What such a product did not compute is NaN.

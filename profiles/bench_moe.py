@@ -2,8 +2,7 @@
 """MoE expert block (quant/switch_linear.py) at the gpt-oss-20b shape: 32 experts, top-4, hidden = inter = 2880, int4 g64.
 
     python profiles/bench_moe.py [--tokens 32]
-Eager timing with CUDA events (the block reads its per-expert row counts back once per call, so it is not graph
-captured); bytes = the packed weights of the experts that were hit (each streamed once) + activations.
+Eager timing with CUDA events of the grouped kernels (six launches, nothing read back); bytes = the packed weights of the experts that were hit (each streamed once) + activations.
 """
 import argparse, json, os, sys
 import torch
@@ -39,6 +38,6 @@ e1.record()
 torch.cuda.synchronize()
 us = e0.elapsed_time(e1) * 1e3 / 20
 wbytes = hit * 3 * (H * I // 2 + 2 * H * I // 64 * 2)
-print(f"tokens={a.tokens} experts hit {hit}/{E} top-{K}: {us:8.1f} us per block, {3 * hit} expert GEMM launches, "
+print(f"tokens={a.tokens} experts hit {hit}/{E} top-{K}: {us:8.1f} us per block, "
       f"{wbytes / 1e6:.1f} MB of expert weights -> {wbytes / us / 1e3:.0f} GB/s ({wbytes / us / 1e3 / peak:.3f} of {peak:.0f})",
       flush=True)

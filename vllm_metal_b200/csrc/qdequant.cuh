@@ -52,6 +52,8 @@ struct Cvt<__half> {
   }
 };
 
+// By mask and magic number: an integer's bits under a chosen exponent read as that power of two plus the integer, which one exact
+// operation takes off again (the method of Kim, Henry, Fahim, Awadalla, "Who Says Elephants Can't Run", 2022, for fp16).
 // 8 nibbles of one packed word -> 8 values s*q+b in memory order (k0..k7), as 4 packed pairs.
 // PRE: the word was nibble-permuted at load time (b200_qlinear_prepack) so that nibbles
 // (i, i+4) hold (k_{2i}, k_{2i+1}); the extraction then yields the pairs in memory order

@@ -12,14 +12,19 @@
 //                          contiguous, however odd K / group is)
 //   1 warp                 the rows of x, by TMA from the grouped fp16 copy
 //   1 warp                 tcgen05.mma, A from tensor memory
+//
+// A result is one chain of K / 16 products in the accumulator, whose additions drop bits: at K = 2880 between 0.1 % (int4) and 0.25 %
+// (int8) of the bf16 results are not the rounding of the float64 sum over the same fp16 weights, as in the dense GEMM above 64 rows.
+// A GEMM of few rows, which splits K, has 0.03 to 0.1 %.  Against the exact weights both are off by the same 0.00166 to 0.0017.
 // A word's nibbles come out as (k_i, k_{i+4}) pairs; the grouped copy holds its columns in that order, so that no permutation
 // of weights is needed, neither at load time nor here.
 //
-// Few rows are bound by the single warps' hand-offs, some 140 cycles each however ready the other side is: a step of 256 columns
-// (SK = 4) instead of 64 and one copy of x for it took a way in of 32 experts of 2880 x 2880, int4, 32 rows in all from 146 to
-// 94 us (its 306 MB of words, scales and biases cross HBM in 47 us); the unpacking warps then work 70 % of the time.  Many rows need the finer ring
-// more (two steps of 128 columns are all that tensor memory has left beside 192 rows): 1024 rows, 183 us with steps of 64
-// columns, 204 with 128; with fast exponentials in the epilogue, whose instructions compete with the unpacking, 169.
+// Few rows are bound by the single warps' hand-offs, whose time does not shrink with the work between them: a step of 256 columns
+// (SK = 4) instead of 64 and one copy of x for it took a way in of 32 experts of 2880 x 2880, int4 in groups of 64, 32 rows in all
+// from 146 to 94 us (words 265 MB, scales and biases 33 MB: 46 us of HBM).  Then 59 % of the issue slots are taken, 38 % of HBM and
+// 8 % of the tensor pipe.  Many rows need the finer ring more (two steps of 128 columns are all that tensor memory has left beside
+// 192 rows): 1024 rows, 183 us with steps of 64 columns, 204 with 128; with fast exponentials in the epilogue, whose instructions
+// compete with the unpacking, 169.  Counters: profiles/expert_products_ncu.txt.
 #include "../../include/b200_hybrid_ops.h"
 #include "qdequant.cuh"
 #include "tcgen05.cuh"
@@ -112,7 +117,8 @@ __device__ __forceinline__ Item item_at(const Params& p, const int* tiles, const
 __device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 __device__ __forceinline__ float clamp_f16(float v) { return fminf(fmaxf(v, -65504.f), 65504.f); }
 
-// Activations of the rounded projections, in fp32.
+// Activations of the rounded projections, in fp32 but for the exponential and the quotient, which are the fast ones: by CUDA's error
+// bounds some 5 + 1.2 |g| last bits (2^-21 near nought, 2^-16 at g = -88), in front of a rounding to the 8 bits of bf16.
 __device__ __forceinline__ float activate(int act, float g, float u) {
   if (act == 1) {  // clipped SwiGLU: alpha 1.702, limit 7
     g = g > 7.f ? 7.f : g;
@@ -554,8 +560,11 @@ weighted_sum_kernel(const __nv_bfloat16* y, const float* weights, __nv_bfloat16*
 // ---- router product and choice --------------------------------------------------------------------------------
 // A block has 16 rows and all experts; its warps split K and add up through shared memory.  A decode step's few blocks are bound
 // by the way to L2, round by round: with WARPS = 32 (16 for more than 32 experts, by registers) 32 x 2880 by
-// 32 experts takes 9.6 us, with 8 warps 20.3.  Products are exact in the accumulator's 32 bits and each warp's chain is K / WARPS long.  Both operands are read in 16-byte pieces, so the columns of a
-// 32-wide step go to the two products in another order than they lie in, the same for both.
+// 32 experts takes 9.6 us, with 8 warps 20.3.  Products are exact; the tensor cores add them up in 32 bits, in chains of
+// K / WARPS.  A logit on the edge between two bf16 values may so go another way than with another order of the sum: of 4096 rows,
+// 9 at 2880 columns by 32 experts have a logit that is not float64's, by an fp32 product with a library 23; 4096 by 64: 13 and 29;
+// 2048 by 128: 4 and 3.  Both operands are read in 16-byte pieces, so the columns of a 32-wide step go to the two products in
+// another order than they lie in, the same for both.
 constexpr int kRouteTop = 32;
 
 template <int NT, int WARPS>  // NT: blocks of 8 experts

@@ -11,10 +11,11 @@
 // of x (UMMA N = NB in {16..256}); the fp32 accumulator [128 x NB] lives in TMEM.
 //
 //   warps 0..DQW-1     dequant: DQW/4 threads per weight row, each unpacks its share of the 64-wide
-//                      k block (int4/int8 -> s*q+b, packed fma, single rounding) -> A ring in the
-//                      canonical K-major SWIZZLE_128B layout
+//                      k block (int4/int8 -> s*q+b, packed fma, single rounding) -> A ring in tensor
+//                      memory (TA); in shared memory, K-major SWIZZLE_128B, only for M <= 64 where scales
+//                      and biases cannot come by TMA, or by the variant knob
 //   warp DQW   (1 thr)  TMA: packed uint32 weight tiles [128 rows x 128 B] -> smem ring (PS deep)
-//   warp DQW+1 (1 thr)  TMA: x tiles [NB x 64] bf16, 128B-swizzled K-major  -> B ring (NS deep)
+//   warp DQW+1 (1 thr)  TMA: x tiles [NB x 64] fp16, 128B-swizzled K-major  -> B ring (NS deep)
 //   warp DQW+2 (1 thr)  tcgen05.mma.cta_group::1.kind::f16 128xNBx16, 4 per 64-wide k block;
 //                      tcgen05.commit frees the A/B stage and finally signals the epilogue
 //   warps 0..DQW-1     epilogue: tcgen05.ld -> (+bias) -> y (warp w reads TMEM lanes 32*(w%4)..)

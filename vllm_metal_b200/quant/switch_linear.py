@@ -8,8 +8,8 @@ expert weights ``[E, N, K*bits/32]`` (third-party arithmetic: mlx 0.32.0 / mlx-l
 
 B200 form: choice of the experts, the sort of the (token, expert) pairs, ONE launch of the gate and up products of all
 experts with the activation in their epilogue, ONE of the down products, the weighted sum (csrc/qexperts.cu).  Nothing is read
-back to the host.  A block of 32 experts of 2880 x 2880, top 4, int4: 172 us for 32 tokens and 313 us for 1024, where a GEMM per
-expert and projection with a read-back of the counts took 1205 and 2745.
+back to the host.  A block of 32 experts of 2880 x 2880, top 4, int4: 159 us for 32 tokens and 313 us for 1024, where a GEMM per
+expert and projection with a read-back of the counts took 1210 and 2734.
 
 Sizes and types that those kernels do not take (``SwitchGLU.grouped_tile_rows``), and the ``mx.gather_qmm`` form of a single
 projection, run one affine quantized GEMM per expert that received rows (`b200_qlinear_experts`), with the row counts read back
@@ -263,7 +263,8 @@ class MoEBlock(nn.Module):
 
     ``routing="topk_softmax"`` (gpt-oss): top-k of the router logits, softmax over the k selected logits.
     ``routing="softmax_topk"`` (Qwen3-MoE style): softmax over all experts, top-k, optionally renormalised.
-    Router and softmax in fp32; ``y = sum_j score_j * expert_j(x)`` accumulated in fp32, rounded once."""
+    Logits are sums of 32 bits rounded to the activations' type, the softmax is in fp32 (the grouped kernels add logits up on the
+    tensor cores and take the activations' exponentials fast); ``y = sum_j score_j * expert_j(x)`` accumulated in fp32, rounded once."""
 
     def __init__(self, router: nn.Module, experts: SwitchGLU, top_k: int, routing: str = "topk_softmax",
                  norm_topk_prob: bool = True) -> None:
