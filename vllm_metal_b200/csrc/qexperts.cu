@@ -13,22 +13,16 @@
 //   1 warp                 the rows of x, by TMA from the grouped fp16 copy
 //   1 warp                 tcgen05.mma, A from tensor memory
 //
-// A result is one chain of K / 16 products in the accumulator, whose additions drop bits: at K = 2880 between 0.1 % (int4) and 0.25 %
-// (int8) of the bf16 results are not the rounding of the float64 sum over the same fp16 weights, as in the dense GEMM above 64 rows.
-// A GEMM of few rows, which splits K, has 0.03 to 0.1 %.  Against the exact weights both are off by the same 0.00166 to 0.0017.
-// A word's nibbles come out as (k_i, k_{i+4}) pairs; the grouped copy holds its columns in that order, so that no permutation
-// of weights is needed, neither at load time nor here.
-//
-// Few rows are bound by the single warps' hand-offs, whose time does not shrink with the work between them: a step of 256 columns
-// (SK = 4) instead of 64 and one copy of x for it took a way in of 32 experts of 2880 x 2880, int4 in groups of 64, 32 rows in all
-// from 146 to 94 us (words 265 MB, scales and biases 33 MB: 46 us of HBM).  Then 59 % of the issue slots are taken, 38 % of HBM and
-// 8 % of the tensor pipe.  Many rows need the finer ring more (two steps of 128 columns are all that tensor memory has left beside
-// 192 rows): 1024 rows, 183 us with steps of 64 columns, 204 with 128; with fast exponentials in the epilogue, whose instructions
-// compete with the unpacking, 169.  Counters: profiles/expert_products_ncu.txt.
+// The accumulators' additions drop bits, the more of them in a chain the more: a result that is one chain of K = 2880 is not the
+// rounding of the float64 sum over the same fp16 weights in 0.13 % (int4) to 0.19 % (int8) of cases, as in the dense GEMM above 64
+// rows; a GEMM of few rows, which splits K, has 0.04 to 0.06 %.  So narrow tiles deal their steps out to four accumulators (two for
+// 64 rows) which the epilogue adds up: 0.04 to 0.06 % (64 rows 0.07 to 0.10).  32 rows 166 -> 168 us a block, 128 rows 168 -> 174.  The
+// sums of every step in registers instead, 0.02 %, took 197 and 201.
 #include "../../include/b200_hybrid_ops.h"
 #include "qdequant.cuh"
 #include "tcgen05.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <mutex>
@@ -56,7 +50,7 @@ struct Params {
   void* out;
   int64_t out_stride;
   int total, experts, n_out, groups, num_kb, max_tiles;
-  int cap, box, ps, nx, na, nbuf, act;
+  int cap, box, ps, nx, na, nbuf, act, chains;
   int* status;  // on the host; set to 1 if a wait ran out or the plan did not fit together
 };
 
@@ -151,7 +145,7 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   volatile int* sfail = reinterpret_cast<volatile int*>(gen + (tmem_ptr - sm_bar) + 4);
   int* tiles = reinterpret_cast<int*>(gen + kBarBytes);
   int* first = tiles + p.experts + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chains = SK == 4 ? p.chains : 1;
   pdl_trigger();
   if (threadIdx.x == 0) {
     for (int i = 0; i < p.ps; ++i) {
@@ -285,13 +279,14 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     // ===== products =====
     const uint32_t tb = __shfl_sync(0xffffffffu, tmem, 0);
     const uint64_t x_desc = make_smem_desc(sm_x);
-    const uint32_t a0 = tb + 2 * p.cap, half = p.cap * 8;  // a 64-column block of x, in the descriptor's units
+    const uint32_t a0 = tb + 2 * chains * p.cap, half = p.cap * 8;  // a 64-column block of x, in the descriptor's units
     int st = 0, xs = 0, it = 0;
     uint32_t ph = 0, xph = 0;
     for (int i = blockIdx.x; ok && i < items; i += gridDim.x, ++it) {
       const Item w = item_at<FEATURES>(p, tiles, first, ft, i);
-      const uint32_t idesc = make_idesc(0, 128, (w.nrows + 15) & ~15), d = tb + (it & 1) * p.cap;
+      const uint32_t idesc = make_idesc(0, 128, (w.nrows + 15) & ~15), d = tb + (it & 1) * chains * p.cap;
       if (!(ok = mbar_wait_or_fail(bar_free + 8 * (it & 1), ((it >> 1) & 1) ^ 1))) break;
+      int chain = 0;
       for (int kb = 0; kb < p.num_kb; kb += SK) {
         // both looked at at once, then waited for what was not ready
         const bool rx = mbar_try_wait(bar_full_x + 8 * xs, xph), ra = mbar_try_wait(bar_full + 8 * st, ph);
@@ -306,7 +301,8 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             if (h == 0 || kb + h < p.num_kb) {
 #pragma unroll
               for (int k = 0; k < 4; ++k)
-                tc_mma_f16_ts(d, a + 32 * h + 8 * k, x + h * half + 2 * k, idesc, h == 0 && k == 0 ? (kb != 0 ? 1u : 0u) : 1u);
+                tc_mma_f16_ts(d + chain * p.cap, a + 32 * h + 8 * k, x + h * half + 2 * k, idesc,
+                              h == 0 && k == 0 ? (kb >= chains * SK ? 1u : 0u) : 1u);
             }
           tc_commit(bar_empty_x + 8 * xs);
           tc_commit(bar_empty + 8 * st);
@@ -315,13 +311,14 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         __syncwarp();
         if (++st == p.na) st = 0, ph ^= 1;
         if (++xs == p.nx) xs = 0, xph ^= 1;
+        if (++chain == chains) chain = 0;
       }
     }
     if (!ok && lane == 0) *sfail = 1;
   } else if (warp < W_EPI) {
     // ===== unpack =====
     const int r = threadIdx.x & 127, hsel = (threadIdx.x >> 7) & 1;
-    const uint32_t xr = r & 7, tm_a = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 2 * p.cap + hsel * 16;
+    const uint32_t xr = r & 7, tm_a = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 2 * chains * p.cap + hsel * 16;
     int pst = 0, it = 0, slot = 0;
     uint32_t pph = 0, sph = 1;
     for (int i = blockIdx.x; ok && i < items; i += gridDim.x, ++it) {
@@ -395,6 +392,7 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     // ===== epilogue: thread = weight row of the tile; the sets of four warps take columns in turn =====
     const int q = warp & 3, r = q * 32 + lane, set = (warp - W_EPI) >> 2;
     const uint32_t tm = tmem + ((uint32_t)(q * 32) << 16);
+    const int used = min(chains, (p.num_kb + SK - 1) / SK);
     int it = 0, flip = 0;
     for (int i = blockIdx.x; i < items; i += gridDim.x, ++it) {
       const Item w = item_at<FEATURES>(p, tiles, first, ft, i);
@@ -410,15 +408,24 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       }
       if (!ok) break;
       tc_fence_after();
-      const uint32_t d = tm + (it & 1) * p.cap;
+      const uint32_t d = tm + (it & 1) * chains * p.cap;
+      auto sums = [&](uint32_t col, uint32_t (&v)[16]) {
+        tmem_ld<16>(d + col, v);
+        for (int j = 1; j < used; ++j) {
+          uint32_t t[16];
+          tmem_ld<16>(d + j * p.cap + col, t);
+#pragma unroll
+          for (int c = 0; c < 16; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) + __uint_as_float(t[c]));
+        }
+      };
       if constexpr (GATED) {
         __half* out = reinterpret_cast<__half*>(p.out);
         for (int c0 = set * 32; c0 < w.nrows; c0 += 32 * kEpiSets) {
           uint32_t mine[16], other[16] = {};
           // gate lanes finish the first 16 columns, up lanes the second: each hands its other 16 over
           const bool second = c0 + 16 < w.nrows;  // the last 32 columns may hold one sixteen only
-          if (second || !which) tmem_ld<16>(d + c0 + which * 16, mine);
-          if (second || which) tmem_ld<16>(d + c0 + (which ? 0 : 16), other);
+          if (second || !which) sums(c0 + which * 16, mine);
+          if (second || which) sums(c0 + (which ? 0 : 16), other);
           const uint32_t ex = sm_ex + set * 8192 + (flip & 1) * 4096;
 #pragma unroll
           for (int c = 0; c < 16; c += 2) {
@@ -456,7 +463,7 @@ expert_qgemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         const bool odd = lane & 1, live = feature < p.n_out;
         for (int c0 = set * 16; c0 < w.nrows; c0 += 16 * kEpiSets) {
           uint32_t u[16];
-          tmem_ld<16>(d + c0, u);
+          sums(c0, u);
           const int place = (int)min((uint32_t)p.pairs[w.row0 + min(c0 + (lane & 15), w.nrows - 1)], (uint32_t)p.total - 1);
 #pragma unroll
           for (int c = 0; c < 16; c += 2) {
@@ -672,6 +679,9 @@ struct Rings {
 constexpr int kCaps[] = {16, 32, 64, 96, 128, 160, kMaxTile};
 constexpr int kNumCaps = 7;
 
+// Accumulators that a result's steps of K go to in turn: what fits beside two steps of A, for tiles whose GEMM split K before.
+static int chains_of(int cap) { return cap <= 32 ? 4 : cap <= 64 ? 2 : 1; }
+
 // Rings beside tiles of `cap` rows: three stages of packed words and the x of two steps (narrow tiles) or four 64-column blocks
 // (wide ones) at least, with the scales of two items if they fit.
 static bool rings_of(Rings& o, int cap, int experts, int k, int group, bool gated) {
@@ -746,7 +756,8 @@ static int launch_steps(const b200_qexpert_product_args& a, const Rings& ring, c
   p.box = box;
   p.ps = ring.ps;
   p.nx = ring.nx;
-  p.na = (512 - 2 * ring.cap) / (32 * SK) < kMaxA ? (512 - 2 * ring.cap) / (32 * SK) : kMaxA;
+  p.chains = chains_of(ring.cap);
+  p.na = std::min((512 - 2 * p.chains * ring.cap) / (32 * SK), kMaxA);
   p.nbuf = ring.nbuf;
   p.act = a.activation;
   p.status = status_word(true);
