@@ -591,7 +591,7 @@ route_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w, const __nv_bfloat16
     const uint4 a = *reinterpret_cast<const uint4*>(x0 + k), b = *reinterpret_cast<const uint4*>(x1 + k);
     uint4 v[NT];
 #pragma unroll
-    for (int n = 0; n < NT; ++n) v[n] = __ldg(reinterpret_cast<const uint4*>(w + (int64_t)min(n * 8 + g, experts - 1) * width + t * 8 + k));
+    for (int n = 0; n < NT; ++n) v[n] = *reinterpret_cast<const uint4*>(w + (int64_t)min(n * 8 + g, experts - 1) * width + t * 8 + k);
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
       asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
