@@ -18,6 +18,16 @@
 // rows; a GEMM of few rows, which splits K, has 0.04 to 0.06 %.  So narrow tiles deal their steps out to four accumulators (two for
 // 64 rows) which the epilogue adds up: 0.04 to 0.06 % (64 rows 0.07 to 0.10).  32 rows 166 -> 168 us a block, 128 rows 168 -> 174.  The
 // sums of every step in registers instead, 0.02 %, took 197 and 201.
+//
+// A word's nibbles come out as (k_i, k_{i+4}) pairs; the grouped copy holds its columns in that order, so that no permutation
+// of weights is needed, neither at load time nor here.
+//
+// Few rows are bound by the single warps' hand-offs, whose time does not shrink with the work between them: a step of 256 columns
+// (SK = 4) instead of 64 and one copy of x for it took a way in of 32 experts of 2880 x 2880, int4 in groups of 64, 32 rows in all
+// from 146 to 94 us (words 265 MB, scales and biases 33 MB: 46 us of HBM).  Then 57 % of the issue slots are taken, 37 % of HBM and
+// 8 % of the tensor pipe.  Many rows need the finer ring more (two steps of 128 columns are all that tensor memory has left beside
+// 192 rows): 1024 rows, 183 us with steps of 64 columns, 204 with 128; with fast exponentials in the epilogue, whose instructions
+// compete with the unpacking, 169.  Counters: profiles/expert_products_ncu.txt.
 #include "../../include/b200_hybrid_ops.h"
 #include "qdequant.cuh"
 #include "tcgen05.cuh"
