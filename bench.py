@@ -44,7 +44,7 @@ METRIC = "decode tok/s (Llama-3.1-8B int4, bs=64)"
 WORKLOAD = "Llama-3.1-8B affine int4 g64 random-init, paged decode bs=64 ctx 4096 block_size 16 (configs[1])"
 MODEL_DESC = "Llama-3.1-8B (random-init, affine int4 g64 incl. lm_head)"
 
-# --config: the other BASELINE.json configs as bench lines (the default, b, is the headline the driver runs).
+# --config: other workloads as bench lines (the default, b, is the headline).
 # name: (preset, batch, ctx, metric, workload, model description, min gpus)
 CONFIGS = {
     "b": (MODEL, BATCH, CTX, METRIC, WORKLOAD, MODEL_DESC, 1),
@@ -564,7 +564,7 @@ def run_b200(args) -> None:
 
     def timed_graph(fn, reps):
         """fn() captured once in a CUDA graph and replayed: the host's launch cost (~20 us per call through
-        ctypes) must not pace kernels that take less than that (it did at TP >= 2 in round 1)."""
+        ctypes) must not pace kernels that take less than that (it did at TP >= 2 once)."""
         for _ in range(3):
             fn()
         torch.cuda.synchronize()
@@ -705,7 +705,7 @@ def main() -> None:
     ap.add_argument("--warmup", type=int, default=5)
     ap.add_argument("--impl", default="b200", choices=["b200", "reference"])
     ap.add_argument("--no-cpu-baseline", action="store_true")
-    ap.add_argument("--config", default="b", choices=sorted(CONFIGS), help="BASELINE.json config (default b = headline)")
+    ap.add_argument("--config", default="b", choices=sorted(CONFIGS), help="workload (default b = headline)")
     ap.add_argument("--hybrid", action="store_true",
                     help="hybrid decoders (latent attention / Mamba-2 / mLSTM) beside the closest transformer of this framework")
     ap.add_argument("--hybrid-sizes", default="s,m", help="sizes of profiles/bench_hybrid.py")

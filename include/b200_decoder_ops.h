@@ -1,6 +1,6 @@
 /*
  * b200_decoder_ops.h -- C-ABI of the ops either side of the hot path
- * (SURVEY.md section 8(f) rows N1-N3): RMSNorm, RoPE, SiLU*mul, greedy argmax.
+ * (RMSNorm, RoPE, SiLU*mul, greedy argmax).
  * In the reference these are MLX built-ins called by the mlx_lm layer code
  * around `sdpa_forward` (attention/impls/sdpa.py:348-368 q/k norm + RoPE,
  * attention/impls/varlen_rope_compat.py:70-82 batched single-token RoPE,
@@ -84,7 +84,7 @@ int b200_advance_decode(int32_t* input_ids, int32_t* positions, int32_t* seq_len
                         const int32_t* sampled, int batch, int max_blocks, int block_size,
                         void* stream);
 
-/* ---- tensor-parallel sum over NVLink peer memory (SURVEY.md section 8(e)) ----------------------
+/* ---- tensor-parallel sum over NVLink peer memory ----------------------
  * The reference runs single-device (vllm_metal/platform.py:524-529); this is the one exchange
  * step the head/column sharding of the path adds: y = sum over ranks of the o_proj / down_proj
  * partial outputs.  One process per GPU; buffers are shared with CUDA IPC.
@@ -133,7 +133,7 @@ int b200_allreduce_add_rmsnorm_push(const void* x, void* residual, const void* w
                                     int hidden, float eps, int dtype, int out_dtype, void* const* box_ptrs,
                                     int64_t box_bytes, void* epoch, int rank, int world, int grid, void* stream);
 
-/* Greedy token of a vocab-parallel head (SURVEY.md section 8(e): lm_head column-parallel over the vocabulary +
+/* Greedy token of a vocab-parallel head (lm_head column-parallel over the vocabulary +
  * a tiny (max, index) exchange instead of gathering logits).  `logits` [rows, shard_vocab] is this rank's slice
  * (global token id = vocab_offset + column); out[r] = index of the first maximum over ALL ranks' slices -- what
  * b200_argmax / mx.argmax (v1/sampling_batch.py:342-348) gives on the gathered row -- identical on every rank.

@@ -1,7 +1,7 @@
 /*
  * b200_paged_ops.h -- C-ABI of the B200-native decode hot path.
  *
- * This is the drop-in boundary "B3" of SURVEY.md section 8(b): every entry
+ * This is the drop-in boundary to the reference: every entry
  * point below replaces one binding of the reference's native module
  * `_paged_ops` (vllm_metal/metal/paged_ops.cpp:1618-1900) or, for the
  * quantized linears, one MLX call the reference makes

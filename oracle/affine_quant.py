@@ -1,7 +1,7 @@
 """CPU oracle: MLX affine int4/int8 group quantisation.  TEST INFRASTRUCTURE ONLY.
 
-The arithmetic lives in a third-party dependency that is NOT under
-``/root/reference``: **mlx == 0.32.0** (``pyproject.toml:36``), functions
+The arithmetic lives in a third-party dependency that is NOT part of
+the reference's tree: **mlx == 0.32.0** (``pyproject.toml:36``), functions
 ``mx.quantize`` / ``mx.dequantize`` / ``mx.quantized_matmul`` and
 ``mlx.nn.QuantizedLinear``; the AWQ repack lives in **mlx-lm @ 254d153**
 (``pyproject.toml:40``, ``mlx_lm.utils._transform_awq_weights``).  MLX is not
@@ -53,7 +53,7 @@ def unpack(w: np.ndarray, bits: int) -> np.ndarray:
 
 
 def quantize(w: np.ndarray, group_size: int = 64, bits: int = 4, dtype: str = "bfloat16"):
-    """MLX ``mx.quantize`` affine mode, restated (SURVEY.md Appendix B).
+    """MLX ``mx.quantize`` affine mode, restated.
 
     Returns ``(w_q uint32 [N, K*bits/32], scales f32 [N, K/g], biases f32 [N, K/g])``
     with scales/biases already rounded to ``dtype``.

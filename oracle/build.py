@@ -6,7 +6,7 @@ translation unit (``vllm_metal/metal/paged_ops.cpp``) that links MLX private
 headers, nanobind and Apple frameworks (Metal, IOKit, CoreFoundation;
 ``vllm_metal/metal/build.py:246-297``) plus Metal shaders that need ``xcrun
 metal``.  None of that exists on Linux: the reference is **unbuildable here** and
-no ``oracle/_ref`` artefact is produced (stated in DESIGN.md).  The CPU baseline
+no ``oracle/_ref`` artefact is produced.  The CPU baseline
 is therefore this C port (``cpu_baseline.kind = "port"``).
 """
 

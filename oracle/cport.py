@@ -1,5 +1,5 @@
 """ctypes front-end of the oracle's C restatement (``oracle/csrc/oracle_cpu.c``).
-TEST / BASELINE INFRASTRUCTURE ONLY (see ``oracle/__init__.py``).
+TEST AND CPU-TIMING INFRASTRUCTURE ONLY (see ``oracle/__init__.py``).
 
 Arrays are NumPy; 16-bit tensors are bf16 bit patterns in ``uint16`` (use
 ``oracle._numeric.bf16_bits`` / ``bf16_from_bits``).

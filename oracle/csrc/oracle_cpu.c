@@ -1,12 +1,12 @@
 /*
- * oracle_cpu.c -- plain-C restatement of the decode hot path.  TEST / BASELINE
- * INFRASTRUCTURE ONLY: used by tests/ as a second checker and by bench.py as the
+ * oracle_cpu.c -- plain-C restatement of the decode hot path.  TEST AND
+ * CPU-TIMING INFRASTRUCTURE ONLY: used by tests/ as a second checker and by bench.py as the
  * timed CPU baseline ("kind": "port").  Never linked into the product library.
  *
  * parity: attention/KV-write/metadata arithmetic is pinned against the reference's
  * fixtures through the NumPy oracle (tests/test_oracle_golden.py compares this file
  * with oracle/*.py); the affine-quantized arithmetic is "parity unpinned" (MLX 0.32.0
- * is a third-party dependency absent from /root/reference, see oracle/affine_quant.py).
+ * is a third-party dependency absent from the reference's tree, see oracle/affine_quant.py).
  *
  * Reference files each function follows:
  *   oracle_reshape_and_cache  vllm_metal/metal/kernels_v2/reshape_and_cache.metal:60-95

@@ -6,7 +6,7 @@ over the selected logits (gpt-oss) or over all experts followed by top-k and ren
 ``mx.gather_qmm`` projections (= ``affine_quant.quantized_matmul`` with that expert's weights), SwiGLU (plain, or
 gpt-oss's clipped form: ``g = min(gate, 7); u = clip(up, +-7); g * sigmoid(1.702 g) * (u + 1)``), score-weighted sum.
 
-The arithmetic lives in third-party code that is NOT under /root/reference (mlx 0.32.0 ``gather_qmm``, mlx-lm 254d153
+The arithmetic lives in third-party code that is NOT in the reference's tree (mlx 0.32.0 ``gather_qmm``, mlx-lm 254d153
 ``switch_layers.py`` / ``gpt_oss.py``), and no reference test holds a vector for it: **parity unpinned**.
 Precision policy as everywhere in the oracle: fp32 arithmetic on dtype-rounded inputs, one rounding per stored tensor.
 """

@@ -4,7 +4,7 @@ Two restatements of the same path:
 
 ``ref_paged_attn``
     Follows the reference's own test oracle line by line
-    (``/root/reference/tools/attention_bench_utils.py:11-62``): gather K/V by
+    (the reference's ``tools/attention_bench_utils.py:11-62``): gather K/V by
     block table, ``q*scale``, fp32 scores, causal ``triu(k=kv-q+1)``, window
     ``not triu(k=kv-(q+W)+1)``, optional softcap, softmax, cast to V dtype, PV.
     Sinks follow the semantics of ``mx.fast.scaled_dot_product_attention(...,

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Paged decode attention alone at a BASELINE decode shape: heuristic split-KV plan vs single pass.
+"""Paged decode attention alone at the headline decode shape: heuristic split-KV plan vs single pass.
 
     python profiles/bench_decode_attn.py [--bs 64 --ctx 4096 --hq 32 --hkv 8 --d 128 --layers 32]
 CUDA graph of `layers` launches over distinct caches (>> L2), CUDA events; GB/s on the algorithmic bytes.

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Tensor-core quantized GEMM (csrc/qgemm_tc.cu) at M >= 256 on the BASELINE layer shapes.
+"""Tensor-core quantized GEMM (csrc/qgemm_tc.cu) at M >= 256 on the served models' layer shapes.
 
     python profiles/bench_gemm_bigm.py [--ms 256,1024,2048,4096]
 x in fp16 (what the norm / SwiGLU producers hand over), weights in the kernel's prepacked layout, CUDA graph of

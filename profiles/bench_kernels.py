@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Per-kernel timing of the decode step's pieces at the headline shapes (Llama-3.1-8B, bs=64).
 
-    python profiles/bench_kernels.py [--sweep] [--m 64] [--out gpurun_out/kernels.json]
+    python profiles/bench_kernels.py [--sweep] [--m 64] [--out kernels.json]
 
 Every kernel is timed with CUDA events over a rotation of distinct buffers whose total size
 exceeds L2 (126 MB), so each launch streams its operands from HBM.  ``--sweep`` runs the tcgen05

@@ -4,8 +4,8 @@
     python profiles/bench_prefill_attn.py [--hq 32 --hkv 4 --d 128] [--chunk 2048] [--offsets 0,2048,6144]
                                           [--decodes 32] [--kernel 0|1|3]
 
-One 2048-token prefill chunk continuing at `offset` + `decodes` decode rows at ctx U[512, 8192] (SURVEY 8(d) cfg c;
-default head counts = Qwen3-32B at TP=2).  CUDA events over 10 launches after 3 warm-ups; flops =
+One 2048-token prefill chunk continuing at `offset` + `decodes` decode rows at ctx U[512, 8192]
+(default head counts = Qwen3-32B at TP=2).  CUDA events over 10 launches after 3 warm-ups; flops =
 4 * D * H_q * sum_i q_i * (ctx_i + (q_i + 1) / 2) (causal), against MEASURED_PEAKS.json bf16_tflops (burst).
 """
 from __future__ import annotations

@@ -6,8 +6,8 @@
 
 CUDA events over a rotation of distinct weight blobs larger than L2 (126 MB), captured in a CUDA graph
 so host launch overhead does not pace the kernels.  Prints achieved GB/s on the algorithmic bytes
-N*K*(bits/8 + 4/g) + (M*K + M*N_out)*2 against MEASURED_PEAKS.json and, with --legacy, the round-1
-kernel (qgemm_tc.cu, MLX layout) beside it.  Tuning evidence; the main numbers are bench.py's.
+N*K*(bits/8 + 4/g) + (M*K + M*N_out)*2 against MEASURED_PEAKS.json and, with --legacy, the cluster
+kernel (qgemm_tc.cu, MLX layout) beside it.  Tuning evidence; the headline numbers are bench.py's.
 """
 
 from __future__ import annotations
@@ -122,7 +122,7 @@ def main():
             yl = torch.empty((m, n), device="cuda", dtype=torch.bfloat16)
             us = time_us(lambda i: ops.quantized_matmul(x, *mlx[i], group_size=g, bits=bits, out=yl), copies)  # x fp16 with --x16: no cast launch
             row["legacy_us"] = us
-            line += f" round-1 kernel: {us:7.2f} us ({(n * k * (bits / 8 + 4 / g) + m * (k + n) * 2) / us / 1e3 / PEAK:4.2f})"
+            line += f" cluster kernel: {us:7.2f} us ({(n * k * (bits / 8 + 4 / g) + m * (k + n) * 2) / us / 1e3 / PEAK:4.2f})"
         if args.trace:
             tr = torch.zeros((148 * 16 + 64 * 8,), dtype=torch.int64, device="cuda")
             ops.set_qstream_trace(tr)

@@ -2,7 +2,7 @@
 
 * ``gpu`` marker: tests that need a real B200.  Everything else runs on CPU.
 * Seeding mirrors the reference's autouse fixture (tests/conftest.py:47-64).
-* ``/root/reference`` is never read here: golden vectors live in tests/golden/.
+* The reference's tree is never read here: golden vectors live in tests/golden/.
 """
 
 from __future__ import annotations

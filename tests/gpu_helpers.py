@@ -9,7 +9,7 @@ from oracle import paged_attention as oattn
 
 TORCH_DT = {"float32": torch.float32, "float16": torch.float16, "bfloat16": torch.bfloat16}
 
-# Tolerances: BASELINE.json north_star for bf16 (2e-2 max-abs / 1e-2 relative); the
+# Tolerances: for bf16 the project's bound (2e-2 max-abs / 1e-2 relative); the
 # reference's own tables for the others (tests/test_split_kv_decode.py:46-50).
 TOL = {"bfloat16": (2e-2, 1e-2), "float16": (1.5e-2, 1e-2), "float32": (1e-3, 1e-3)}
 

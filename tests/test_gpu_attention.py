@@ -61,7 +61,7 @@ def test_reshape_and_cache_skips_negative_and_out_of_range_slots(ops):
 
 
 def test_reshape_and_cache_full_size_roundtrip(ops):
-    """BASELINE config b row shape (8 kv heads x 128, bf16), 64 decode tokens into a
+    """The headline decode row shape (8 kv heads x 128, bf16), 64 decode tokens into a
     16k-block pool: every written row reads back bit-exact, nothing else changes."""
     h, d, bs, nb, t = 8, 128, 16, 16384, 64
     g = torch.Generator(device="cuda").manual_seed(1)
@@ -300,7 +300,7 @@ def test_sinks_validation(ops):
 # ------------------------------------------------------ full-size properties
 
 def test_full_size_decode_properties(ops):
-    """BASELINE config b shape (bs 64, ctx 4096, 32q/8kv/128, block 16) — too big for the
+    """The headline decode shape (bs 64, ctx 4096, 32q/8kv/128, block 16) — too big for the
     NumPy oracle in seconds, so check (1) 4 sampled sequences against the oracle,
     (2) split-KV == single pass, (3) MMA kernel == generic kernel, (4) linearity in V."""
     seqs = [(1, 4096 + (i % 7)) for i in range(64)]

@@ -1,4 +1,4 @@
-"""Parity at the layer shapes BASELINE.json names (configs[2..4]), not just toy sizes.
+"""Parity at the layer shapes of the served models, not just toy sizes.
 
 * every linear of Qwen3-32B (int8 g64, K = 5120 / 8192 / 25600), Llama-3.1-70B (int4 g64,
   K = 8192 / 28672, and the TP=8 row-parallel shards K = 1024 / 3584) and gpt-oss-20b attention
@@ -7,7 +7,7 @@
 * one Qwen3-32B-shaped layer and a gpt-oss-shaped sliding+full layer pair end to end
   (prefill chunk + decode rows, sinks, window 128, bs 32) against ``OracleDecoder``.
 
-Tolerance: north-star bf16 bound, 2e-2 max-abs + 1e-2 relative.
+Tolerance: the project's bf16 bound, 2e-2 max-abs + 1e-2 relative.
 """
 
 from __future__ import annotations

@@ -117,13 +117,13 @@ def _bf16_ulp(x: float) -> float:
 
 
 def test_cfg_a_qwen3_0p6b_128_free_running_greedy_steps():
-    """BASELINE configs[0] at its stated size: Qwen3-0.6B shapes (28 layers, hidden 1024, 16q/8kv x 128,
+    """At its stated size: Qwen3-0.6B shapes (28 layers, hidden 1024, 16q/8kv x 128,
     vocab 151936, q/k norm, tied int4 g64 head), bs 1, 512-token prompt, block 16, 128 greedy
     decode steps.  The product runs FREE (CUDA graph, its own tokens fed back, as in
-    /root/reference/tests/test_paged_deterministic.py:50-74); the oracle is stepped along the
+    the reference's tests/test_paged_deterministic.py:50-74); the oracle is stepped along the
     product's trajectory and must name the same token at every step.  A differing token is only
     tolerated -- and printed -- when the oracle's own logits of the two candidates are closer than the
-    north-star parity bound on those logits themselves (2e-2 max-abs + 1e-2 relative: they are bf16
+    parity bound on those logits themselves (2e-2 max-abs + 1e-2 relative: they are bf16
     GEMM outputs over 28 layers of bf16 activations, the product accumulates in other orders --
     tensor-core tiles, cluster split-K, stream-K pieces -- than the oracle's fp32 loop, so a candidate's
     logit may legitimately land a couple of bf16 ulps (1 ulp = 0.0156 at |logit| in [1, 2)) away).  With
@@ -142,7 +142,7 @@ def test_cfg_a_qwen3_0p6b_128_free_running_greedy_steps():
     cache = B200PagedKVCache(args.num_layers, args.n_kv_heads, args.head_dim, nb, bs, torch.bfloat16, "cuda")
     runner = PagedModelRunner(model, cache, max_batch=1, max_model_len=blocks * bs, use_cuda_graph=True)
     oracle = oracle_from_model(model, nb, bs)
-    rng = np.random.default_rng(1)  # SURVEY 8(d): token ids seed 1, page permutation seed 2
+    rng = np.random.default_rng(1)  # token ids seed 1, page permutation seed 2
     prompt = rng.integers(0, args.vocab, prompt_len).tolist()
     table = (np.random.default_rng(2).permutation(nb - 1) + 1).tolist()
 

@@ -1,4 +1,4 @@
-"""Quantized MoE expert path (SURVEY.md 8(f) N2) through the C-ABI linears vs oracle/moe.py."""
+"""Quantized MoE expert path through the C-ABI linears vs oracle/moe.py."""
 
 from __future__ import annotations
 
@@ -24,7 +24,7 @@ def _build(hidden, inter, experts, top_k, bits, group, bias, act, routing, seed)
     rnd = lambda *s: torch.randn(s, device="cuda", generator=g)  # noqa: E731
     glu = SwitchGLU(hidden, inter, experts, bias, group, bits, torch.bfloat16, "cuda", activation=act)
     for name, (n, k) in (("gate_proj", (inter, hidden)), ("up_proj", (inter, hidden)), ("down_proj", (hidden, inter))):
-        dense = rnd(experts, n, k) * (0.7 / k ** 0.5)  # activations stay O(1): the bound is the linears' north-star tolerance
+        dense = rnd(experts, n, k) * (0.7 / k ** 0.5)  # activations stay O(1): the bound is the linears' tolerance
         b = rnd(experts, n) * 0.1 if bias else None
         setattr(glu, name, QuantizedSwitchLinear.from_dense(dense, b, group, bits, torch.bfloat16))
     router = torch.nn.Linear(hidden, experts, bias=bias, device="cuda", dtype=torch.bfloat16).requires_grad_(False)
@@ -52,7 +52,7 @@ def test_moe_block_vs_oracle(bits, group, act, routing, bias, tokens):
                                       top_k, group, bits, "bfloat16", routing, act)
     same = [set(a) == set(b) for a, b in zip(idx.cpu().tolist(), oidx.tolist(), strict=True)]
     assert np.mean(same) >= 0.95  # a bf16-rounded logit pair can swap at the k-th place
-    # expert path parity on the product's routing: north-star bound of the quantized linears
+    # expert path parity on the product's routing: bound of the quantized linears
     want, _, _ = omoe.moe_block(to_np(x), rw, rb, _stack(glu.gate_proj), _stack(glu.up_proj), _stack(glu.down_proj),
                                 top_k, group, bits, "bfloat16", routing, act,
                                 indices=idx.cpu().numpy(), scores=scores.cpu().numpy())

@@ -1,7 +1,7 @@
 """GPU parity: MLX-affine quantized linears + decoder neighbours vs the oracle.
 
 Bit-exact: int4/int8 unpack -> dequantised values (``dequantize``).  Within the
-north-star tolerance (2e-2 max-abs / 1e-2 relative, bf16): quantized matmul.
+tolerance (2e-2 max-abs / 1e-2 relative, bf16): quantized matmul.
 Reference anchors: gguf/mlx_native.py:212-239, tests/test_gguf_mlx_native.py:70-86.
 """
 

@@ -2,7 +2,7 @@
 
 Reference anchors: mx.quantized_matmul as called from gguf/mlx_native.py:212-222 and
 nn.QuantizedLinear (attention/impls/sdpa.py:297-343,739); SwiGLU fusion = compiled_mlp.py:1-22.
-Bar: 2e-2 max-abs + 1e-2 relative (north star, bf16 outputs); the integer part of the streaming
+Bar: 2e-2 max-abs + 1e-2 relative (bf16 outputs); the integer part of the streaming
 layout round-trips bit-exactly; results are identical for every persistent-grid size that cuts the
 super-tiles differently (the finisher adds partials in k order, never in arrival order).
 """
@@ -65,7 +65,7 @@ def test_qstream_vs_oracle(ops, m, bits, group):
     (136, 192, 4, 64, 5), (1000, 2048, 4, 128, 33), (384, 1536, 8, 64, 64), (5120, 25600, 8, 64, 64),
     (8192, 28672, 4, 64, 16), (151936, 1024, 4, 64, 1), (128, 2880, 4, 32, 8), (1280, 8192, 4, 64, 16)])
 def test_qstream_model_shapes(ops, n, k, bits, group, m):
-    """Projection shapes of the BASELINE models incl. ragged N (not a multiple of 256), K = 2880 = 22.5 slabs,
+    """Projection shapes of the served models incl. ragged N (not a multiple of 256), K = 2880 = 22.5 slabs,
     the long-K cases (25600 int8, 28672 int4) and the Qwen3-0.6B tied head; oracle on a row subset."""
     gen = torch.Generator(device="cuda").manual_seed(n + k)
     w = torch.randint(-2**31, 2**31 - 1, (n, k * bits // 32), dtype=torch.int64, device="cuda", generator=gen).to(torch.int32)

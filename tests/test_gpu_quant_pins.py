@@ -5,11 +5,11 @@ the only reference-held anchors for rows a13-a15 are these two test files; both 
 here with their tolerances unchanged and their synthetic inputs regenerated from the same
 seeds:
 
-* ``/root/reference/tests/quant/test_awq_repack_parity.py:100-176`` -- an AutoAWQ triple
+* the reference's ``tests/quant/test_awq_repack_parity.py:100-176`` -- an AutoAWQ triple
   (seed 42; ``W = (q - z) * s``) goes through the product's AWQ transform and
   ``b200_dequantize_rows``; max error <= ``max(max|W| * 2**-9, 2e-3)``, mean < a quarter of it,
   shapes ``weight [out, in/8]`` uint32, ``scales/biases [out, in/128]``.
-* ``/root/reference/tests/test_gguf_mlx_native.py:70-86`` -- group-32 ``matmul`` with float32
+* the reference's ``tests/test_gguf_mlx_native.py:70-86`` -- group-32 ``matmul`` with float32
   activations against the dense dequantised oracle at ``atol = max|ref| * 4e-6``; output dtype
   follows ``x`` (:89-99); leading dims preserved (:102-110).
 """

@@ -66,7 +66,7 @@ def test_windowed_matches_expanded(ops, dtype, hq, hkv, ctx, window):
 @pytest.mark.parametrize("hq,hkv", [(16, 8), (32, 8), (8, 8), (64, 8)])
 @pytest.mark.parametrize("ctx", [512, 8192])
 def test_windowed_matches_oracle(ops, dtype, hq, hkv, ctx):
-    """:197-242, against the CPU oracle with the north-star tolerance."""
+    """:197-242, against the CPU oracle with the bf16 tolerance."""
     _, windowed, c = _expanded_and_windowed(ops, hq, hkv, dtype, ctx, [5, 1, 3], -1, seed=2)
     assert_close(windowed, oracle_attention(c), dtype, f"window mode {hq}q/{hkv}kv ctx {ctx}")
 

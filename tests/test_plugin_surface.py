@@ -1,4 +1,4 @@
-"""Host-side plugin surface (B1 platform, B2 worker, quant-method hook) on CPU.
+"""Host-side plugin surface (platform, worker, quant-method hook) on CPU.
 
 These mirror what the reference's own tests check about its plugin layer without a device
 (tests/test_platform.py, tests/test_block_size_translation.py): entry points resolve, the

@@ -1,4 +1,4 @@
-"""Tensor-parallel host logic on CPU with a real world-size-2 ``gloo`` group (SURVEY.md 8e).
+"""Tensor-parallel host logic on CPU with a real world-size-2 ``gloo`` group.
 
 Two processes shard one quantized attention/MLP block the way ``lm/decoder.py`` does
 (column-parallel q/k/v + gate/up via ``shard_rows``, row-parallel o_proj/down via ``shard_cols``),

@@ -1,7 +1,7 @@
 // One-shot sum all-reduce over NVLink peer memory for the tensor-parallel decode step.
 //
 // The reference has no tensor parallelism (vllm_metal/platform.py:524-529 pins world size 1);
-// SURVEY.md 8(e) shards this path over heads / MLP columns, which leaves one [M, hidden] sum after
+// here this path is sharded over heads / MLP columns, which leaves one [M, hidden] sum after
 // o_proj and one after down_proj per layer -- 512 KiB at the headline shape, far below the size
 // where a ring pays, and latency-bound in NCCL (~20 us each, 64 per step).  This kernel does the
 // exchange itself through CUDA-IPC mapped peer buffers (NVSwitch gives every pair full bandwidth):
@@ -131,7 +131,7 @@ static int launch(const Params& p, int grid, cudaStream_t st) {
 
 // ---- fused: all-reduce + residual add + RMSNorm ------------------------------------------------------------
 // The two sums of a tensor-parallel decoder layer are each followed by `h += sum; x = rms_norm(h) * w`
-// (reference layer wiring; SURVEY.md 8(e) asks for the fused form).  CTA b owns ROWS b, b + grid, ... on every
+// (reference layer wiring).  CTA b owns ROWS b, b + grid, ... on every
 // rank (a row of the headline shape is 8 KiB: one 16-byte vector per thread), so after the same flag exchange as
 // above it gathers a whole row from every peer, adds in rank order, rounds the sum to T exactly as the unfused
 // all-reduce stores it, adds the residual (rounded to T, as b200_rms_norm does), keeps the row in registers for
@@ -524,7 +524,7 @@ static int launch_ll(const LLParams& f, int grid, cudaStream_t st) {
   return check_launch("allreduce_add_rmsnorm_ll_kernel");
 }
 
-// ---- vocab-parallel greedy head: (max logit, token) exchange (lm_head row) ----------------
+// ---- vocab-parallel greedy head: (max logit, token) exchange ----------------
 // Every rank holds the logits of its own vocab slice; the greedy token is the arg-max over all slices.  Each rank
 // PUSHES its per-row winner (value, global index) into every peer's slot table with two 8-byte stores that carry
 // the call's epoch in their upper word (NCCL's LL idea: the data is its own flag, no separate signal and no fence),

@@ -4,7 +4,7 @@
 
 namespace b200 {
 
-// Split-KV scratch layout (fp32 partials; SURVEY.md appendix A.4 -- the
+// Split-KV scratch layout (fp32 partials -- the
 // reference keeps tmp_out in the query dtype, paged_ops.cpp:647-653):
 //   tmp_out  float [T, H_q, P, D]   un-normalised partial numerators
 //   max_l2   float [T, H_q, P]      running max in the log2 domain

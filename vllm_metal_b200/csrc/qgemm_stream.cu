@@ -8,7 +8,7 @@
 // attention/impls/sdpa.py:297-343,739; the SwiGLU the reference fuses in compiled_mlp.py:1-22).
 //
 // Why a second kernel next to qgemm_tc.cu: at M <= 64 the op is a weight stream (HBM-bound), and
-// round 1's one-CTA-per-row-tile kernel spent it on per-CTA prologue/epilogue, a 0.76-wave grid and
+// a one-CTA-per-row-tile kernel spent it on per-CTA prologue/epilogue, a 0.76-wave grid and
 // one mbarrier hand-off per 64 k.  Here:
 //
 //   * ONE persistent CTA per SM.  The (row super-tile x k-slab) units of the matrix are cut into
@@ -859,7 +859,7 @@ __global__ void qstream_unpack_kernel(const PackParams p, uint32_t* out) {
 
 // bf16 -> fp16 for the B operand.  Exact for every bf16 whose magnitude is a normal fp16 (8 significant bits fit
 // in 11); magnitudes above 65504 saturate (bf16 activations of that size do not occur after a norm / SwiGLU; the
-// reference would carry them, this path clamps -- stated in DESIGN.md), below 2^-24 round to zero.
+// reference would carry them, this path clamps), below 2^-24 round to zero.
 __global__ void cast_bf16_f16_sat_kernel(const __nv_bfloat16* __restrict__ x, __half* __restrict__ y, int rows, int cols,
                                          int64_t x_stride) {
   pdl_trigger();

@@ -1,4 +1,4 @@
-// Fused per-head RMSNorm -> RoPE -> KV-cache write (SURVEY.md section 8(f) row N1).
+// Fused per-head RMSNorm -> RoPE -> KV-cache write.
 //
 // One launch does what the reference's sdpa_forward does in five steps between the q/k/v
 // projections and the attention kernel (vllm_metal/attention/impls/sdpa.py:348-368 q/k norm +

@@ -1,4 +1,4 @@
-"""Tensor-parallel sum over NVLink peer memory (SURVEY.md 8(e); kernel: csrc/nvlink_allreduce.cu).
+"""Tensor-parallel sum over NVLink peer memory (kernel: csrc/nvlink_allreduce.cu).
 
 ``torch.distributed`` is the plumbing only (rank/world, one ``all_gather_object`` of the CUDA-IPC
 handles at construction); the per-layer exchange is our own one-shot kernel through peer-mapped

@@ -8,7 +8,7 @@ packed ``qkv_proj``, ``n_heads``, ``n_kv_heads``, ``scale``, ``q_norm``/
 ``k_norm``, ``rope``, ``sinks``) so ``sdpa_forward`` duck-types it identically.
 Weights are MLX-affine quantized (``QuantizedLinear``); tensor parallelism shards
 heads / MLP columns per rank and sums o_proj / down_proj outputs with an
-allreduce (SURVEY.md section 8(e)).
+allreduce.
 """
 
 from __future__ import annotations
@@ -210,7 +210,7 @@ class Model(nn.Module):
         self.args = args
         self.rank, self.world = rank, world
         self._allreduce = allreduce
-        # Vocab-parallel head (SURVEY 8(e)): each rank keeps vocab / world rows of the head and the greedy token comes
+        # Vocab-parallel head: each rank keeps vocab / world rows of the head and the greedy token comes
         # from a (max, id) exchange (``greedy``); ``forward`` then returns this rank's logits slice only.
         if vocab_parallel is None:
             vocab_parallel = world > 1 and hasattr(allreduce, "argmax_vocab_parallel") and args.vocab % world == 0

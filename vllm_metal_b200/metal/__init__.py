@@ -224,7 +224,7 @@ def load_library() -> ctypes.CDLL:
     if os.environ.get("VLLM_METAL_BUILD_FROM_SOURCE", "0") not in ("", "0"):
         build()
     so = output_path()
-    override = os.environ.get("B200_PAGED_OPS_LIB")  # tuning experiments only (profiles/build_variants.sh)
+    override = os.environ.get("B200_PAGED_OPS_LIB")  # tuning experiments only
     if override:
         from pathlib import Path
 

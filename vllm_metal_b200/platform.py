@@ -1,11 +1,11 @@
-"""vLLM platform plugin for the B200 decode path (boundary B1).
+"""vLLM platform plugin for the B200 decode path.
 
 Mirrors the hooks ``vllm_metal/platform.py:25-1022`` overrides -- device queries, request
 validation, config gates, worker class, block-size hook, synthetic attention backend -- with the
 device being ``cuda:<local_rank>`` of compute capability 10.x instead of the single Apple GPU.
 Only host-side glue: no kernels are launched from here.  What the reference's platform does for
 Ray / MLX wired memory / hybrid-model TurboQuant realignment is outside the hot path and is not
-reproduced (DESIGN.md "out of scope").
+reproduced.
 """
 
 from __future__ import annotations

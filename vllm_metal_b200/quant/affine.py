@@ -1,6 +1,6 @@
 """MLX affine group quantisation in torch (load-time helper).
 
-Restates ``mx.quantize`` (MLX 0.32, third-party; SURVEY.md appendix B) so
+Restates ``mx.quantize`` (MLX 0.32, third-party) so
 random-init or dense checkpoints can be turned into the MLX triple
 ``weight`` (uint32 bit patterns stored as int32) / ``scales`` / ``biases``.
 Runs on whatever device the weight lives on; it is load-time code, not part of

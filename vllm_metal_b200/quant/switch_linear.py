@@ -1,10 +1,10 @@
-"""Quantized mixture-of-experts MLP (SURVEY.md 8(f) N2): ``QuantizedSwitchLinear`` / ``SwitchGLU`` / ``MoEBlock``.
+"""Quantized mixture-of-experts MLP: ``QuantizedSwitchLinear`` / ``SwitchGLU`` / ``MoEBlock``.
 
 The reference reaches MoE models (gpt-oss: 32 experts, top-4) through mlx-lm's ``SwitchGLU`` whose expert
 projections are ``QuantizedSwitchLinear`` modules -- named in vllm_metal/quant/awq_loader.py:171-173 -- i.e.
 ``mx.gather_qmm(x, weight, scales, biases, rhs_indices=indices, transpose=True, group_size, bits)`` over stacked
-expert weights ``[E, N, K*bits/32]`` (third-party arithmetic: mlx 0.32.0 / mlx-lm 254d153, not under
-/root/reference -> parity unpinned, semantics restated in oracle/moe.py).  Same attribute names and shapes here.
+expert weights ``[E, N, K*bits/32]`` (third-party arithmetic: mlx 0.32.0 / mlx-lm 254d153, not in
+the reference's tree -> parity unpinned, semantics restated in oracle/moe.py).  Same attribute names and shapes here.
 
 B200 form: choice of the experts, the sort of the (token, expert) pairs, ONE launch of the gate and up products of all
 experts with the activation in their epilogue, ONE of the down products, the weighted sum (csrc/qexperts.cu).  Nothing is read

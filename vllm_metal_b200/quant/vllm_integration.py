@@ -23,7 +23,7 @@ NAME = "mlx_affine"
 
 class MLXAffineConfig(QuantizationConfig):
     """``{"quantization": {"group_size": 32|64|128, "bits": 4|8}}`` as mlx-lm writes it into
-    ``config.json`` (SURVEY.md Appendix B).  Lives at module top level: it is pickled into the
+    ``config.json``.  Lives at module top level: it is pickled into the
     EngineCore / worker processes."""
 
     _SUPPORTED_ACT_DTYPES = [torch.bfloat16, torch.float16]

@@ -1,4 +1,4 @@
-"""One-step-ahead decode pipelining for the B200 worker (SURVEY.md 8(f) N4, "deferred sampling").
+"""One-step-ahead decode pipelining for the B200 worker ("deferred sampling").
 
 Reference: vllm_metal/v1/decode_pipeline.py:1-26, 182-347.  A fully serial decode step launches the step, then blocks
 on the sampled tokens while the GPU idles through the next step's host work.  Here step ``k`` is submitted without

@@ -1,4 +1,4 @@
-"""Speculative decoding around the paged decode path (SURVEY.md 8(f) N4): greedy verification of scheduled draft
+"""Speculative decoding around the paged decode path: greedy verification of scheduled draft
 tokens and a prompt-lookup (n-gram) drafter.
 
 The reference verifies a K+1-row window per request with the target model's greedy tokens

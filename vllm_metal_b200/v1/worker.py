@@ -1,4 +1,4 @@
-"""vLLM worker for the B200 decode path (boundary B2).
+"""vLLM worker for the B200 decode path.
 
 Mirrors the method set of ``MetalWorker(WorkerBase)`` (vllm_metal/v1/worker.py:65-404): device
 init, model load, KV-cache sizing/spec/initialisation, ``execute_model`` -> ``sample_tokens``.
@@ -7,7 +7,7 @@ The engine-side scheduler drives it; everything on the device goes through
 greedy decode + chunked-prefill contract of the hot path is implemented, plus greedy verification of
 scheduled draft tokens in the decode kernel's window mode with a prompt-lookup drafter
 (``v1/spec_decode.py``): LoRA, multimodal, model-based drafters, sleep mode and pipeline parallelism
-raise or no-op exactly where the reference's worker has its own gates (DESIGN.md "out of scope").
+raise or no-op exactly where the reference's worker has its own gates.
 """
 
 from __future__ import annotations
@@ -102,7 +102,7 @@ class B200Worker(WorkerBase):
 
     def load_model(self) -> None:
         """Builds the decoder for the HF config with RANDOM-INITIALISED affine-quantized weights (``seed``):
-        the BASELINE configs are all random-init and no checkpoint reader is wired for these families (the AWQ repack
+        the benchmarked configurations are all random-init and no checkpoint reader is wired for these families (the AWQ repack
         path is ``quant/awq_loader.py``; hybrid decoders do load safetensors).  ``load_format`` other than
         "dummy"/"auto" therefore raises instead of silently ignoring a checkpoint."""
         lf = str(getattr(getattr(self.vllm_config, "load_config", None), "load_format", "dummy"))
